@@ -256,9 +256,12 @@ int grid_for(HyCtx* c, int mode, bool count, int minb, bool short_stack, int sha
     return per * c->num_sms;
 }
 
-// tile streams: node visits per scheduling round (1080p shadow kernel at 8
-// resident blocks over the SAH structure: 8 / 12 / 16 visits 22.8 / 22.5 / 23.2 ms)
-constexpr uint32_t kStreamSteps = 12;
+// tile streams: node visits per scheduling round.  A round ends with the test of
+// the triangles it reached, so short rounds cost little and leave fewer lanes
+// walking on behind an occluder: shadow kernel at 3 / 4 / 6 / 8 / 12 visits, 1080p x
+// 16 spp 18.25 / 17.88 / 17.83 / 17.86 / 18.23 ms, 4K x 64 lights 144.1 / 143.1 /
+// 146.6 / 149.2 / 161.0 ms, 1277x719 two-level 13.5 / 13.0 / 13.0 / 13.2 / 13.7 ms
+constexpr uint32_t kStreamSteps = 4;
 
 PassParams make_params(HyCtx* c, const HyGBuffer* gb, const HyCamera* cam, const HyPassConfig* cfg,
                        uint32_t accum_fmt, void* shadow, void* hist, float* out_f, uint8_t* out_8) {
@@ -293,8 +296,7 @@ PassParams make_params(HyCtx* c, const HyGBuffer* gb, const HyCamera* cam, const
     P.chunk = cfg->queue_chunk ? cfg->queue_chunk : 1;
     // node visits per scheduling round of the persistent shadow kernels: 4
     // measured 9.5 % ahead of 1 for the lane groups on the 1080p workload
-    // (2: 6.8 %, 3: 8.8 %, 8: 8.9 %); the tile streams default to 8 (at 8
-    // resident blocks: 4: -3.9 %, 6: -1.7 %, 12: -3.6 %, 16: -2.7 %)
+    // (2: 6.8 %, 3: 8.8 %, 8: 8.9 %); the tile streams: kStreamSteps
     P.inner = cfg->visits_per_round ? std::min(cfg->visits_per_round, 16u) : 4u;
     if (cfg->flags & HY_FLAG_FULL_BLUR_DISPATCH) { P.blur_w = P.W; P.blur_h = P.H; }
     else { P.blur_w = (P.W / 16) * 16; P.blur_h = (P.H / 16) * 16; }
@@ -370,8 +372,7 @@ int run_pixels(HyCtx* c, int mode, const PassParams& P0, const HyPassConfig* cfg
         }
     }
     // measured fastest on the 1080p workload: 6 resident blocks (80 registers)
-    // for the lane-group kernel (1.4 % ahead of 8), 8 (64 registers) otherwise;
-    // 12 node visits per round for the tile streams (4 for the others)
+    // for the lane-group kernel (1.4 % ahead of 8), 8 (64 registers) otherwise
     const bool grouped = mode == MODE_SHADOW_G || mode == MODE_SHADOW_ACCUM_G;
     const bool streams = mode == MODE_SHADOW_S || mode == MODE_SHADOW_ACCUM_S;
     int minb = cfg->min_blocks ? (int)cfg->min_blocks : (grouped ? 6 : 8);

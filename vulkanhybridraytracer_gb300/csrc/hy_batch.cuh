@@ -24,8 +24,10 @@ namespace hy {
 static_assert(sizeof(PassParams) % 4 == 0 && sizeof(SceneDev) % 4 == 0, "copied to shared memory as words");
 template <bool COUNT, int BLOCK, int MINB, int SHORT, bool ANY_TWO>
 __global__ void __launch_bounds__(BLOCK, MINB) k_shadow_batch_stream(const BatchParams B) {
+    static_assert(!ANY_TWO || (BLOCK == 128 && SHORT == 0), "two-level views: one launch shape");
     constexpr int NW = BLOCK / 32;
-    __shared__ StreamSlotsT<NW> sm;
+    __shared__ StreamSlotsT<NW, ANY_TWO> sm;
+    __shared__ float s_world[ANY_TWO ? 6 * BLOCK : 1];  // two-level views: WorldRaySlot words
     // per warp: its current view's parameters and scene, copied from the
     // global tables when the warp moves to another view
     __shared__ PassParams s_view[NW];
@@ -64,22 +66,19 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_shadow_batch_stream(const Batch
         const SceneDev& S = s_scene[warp];
         const bool accum = !(P.flags & HY_FLAG_NO_ACCUM) && P.accum_frame > 0;
         const bool reference = P.rng_mode == HY_RNG_REFERENCE;
-        if constexpr (SHORT > 0) {
-            const SplitStackT<SHORT, BLOCK> sst{s_stack + threadIdx.x, stk};
-            if (ANY_TWO && S.two_level)
-                stream_tile<COUNT, true, 2>(S, P, unit - P.tile_begin, reference, accum, sm, sst, t, r, s, ls, nn, nt,
-                                            nullptr, 0);
-            else
-                stream_tile<COUNT, false, 2>(S, P, unit - P.tile_begin, reference, accum, sm, sst, t, r, s, ls, nn,
-                                             nt, nullptr, 0);
-        } else {
-            if (ANY_TWO && S.two_level)  // a two-level scene: the same tile with the instance walk
-                stream_tile<COUNT, true, 2>(S, P, unit - P.tile_begin, reference, accum, sm, stk, t, r, s, ls, nn, nt,
-                                            nullptr, 0);
-            else
-                stream_tile<COUNT, false, 2>(S, P, unit - P.tile_begin, reference, accum, sm, stk, t, r, s, ls, nn,
-                                             nt, nullptr, 0);
+        const uint32_t tile = unit - P.tile_begin;
+        if constexpr (ANY_TWO) {  // compiled without a shared stack
+            if (S.two_level) {
+                WorldRaySlot w{s_world + threadIdx.x, &sm.scratch[warp].walk.ray[lane]};
+                stream_tile<COUNT, true, 2>(S, P, tile, reference, accum, sm, stk, t, w, s, ls, nn, nt);
+                continue;
+            }
         }
+        if constexpr (SHORT > 0)
+            stream_tile<COUNT, false, 2>(S, P, tile, reference, accum, sm,
+                                         SplitStackT<SHORT, BLOCK>{s_stack + threadIdx.x, stk}, t, r, s, ls, nn, nt);
+        else
+            stream_tile<COUNT, false, 2>(S, P, tile, reference, accum, sm, stk, t, r, s, ls, nn, nt);
     }
     if (COUNT) { ls.nodes += nn; ls.tris += nt; }
     flush_stats(ls, B.stats);

@@ -447,6 +447,13 @@ __device__ __forceinline__ uint2 stack_get(const SplitStackT<SH, STRIDE>& s, int
     return i < SH ? s.sh[i * STRIDE] : s.deep[i - SH];
 }
 
+// Where a walk reports a limit that ran out: the call's status word, or a
+// register of a caller that first has to know whether the ray was hit before
+// its walk reached the limit.
+struct DeferredStatus { uint32_t& bits; };
+__device__ __forceinline__ void raise_status(uint32_t* s, uint32_t f) { atomicOr(s, f); }
+__device__ __forceinline__ void raise_status(DeferredStatus s, uint32_t f) { s.bits |= f; }
+
 // Stack traversal of the 8-wide BVH.  ANY: TerminateOnFirstHit semantics.
 // COUNT: accumulate node visits / triangle tests.
 //
@@ -474,6 +481,7 @@ struct Trav {
     RayPre cur;                  // the ray in the frame of the level being walked
     uint32_t inst_base, inst_bits;  // hit instance entries of the last TLAS leaf set
     uint32_t id_off;             // first global triangle of the instance being walked
+    uint32_t inst;               // the instance being walked
     int sp_base;                 // stack height when the instance was entered
     bool level;                  // inside a BLAS
 };
@@ -491,6 +499,7 @@ __device__ __forceinline__ void trav_init(Trav& t, const RayPre& r, float tmax) 
     t.inst_base = 0;
     t.inst_bits = 0;
     t.id_off = 0;
+    t.inst = 0;
     t.sp_base = 0;
     t.level = false;
 }
@@ -516,14 +525,13 @@ __device__ __forceinline__ f3 xform_dir(float4 r0, float4 r1, float4 r2, f3 d) {
 }
 
 // A lane's world ray: its set-up in registers (RayPre), or, for the two-level
-// walk, in shared memory (WorldRaySlot: word k of lane t at p[128 k], the 16
-// words of RayPre, conflict-free; 64 B a lane).  The two-level walk reads the
-// world ray only to enter and leave instances, so its registers go to the walk.
-// (Keeping only the origin and direction there and recomputing the set-up on
-// leaving an instance freed more shared memory for L1 but made the 4K two-level
-// frame slower: 293.4 against 282 ms.)
+// walk of the tile streams, in shared memory (WorldRaySlot: the direction and
+// tmax in the lane's float4, word k of the origin and the reciprocal direction
+// at p[128 k], conflict-free).  The two-level walk reads the world ray only to
+// enter and leave instances, so its registers go to the walk.
 struct WorldRaySlot {
     float* p;
+    float4* ray;
 };
 __device__ __forceinline__ f3 world_o(const RayPre& r) { return r.o; }
 __device__ __forceinline__ f3 world_d(const RayPre& r) { return mk(r.d[0], r.d[1], r.d[2]); }
@@ -533,25 +541,20 @@ __device__ __forceinline__ const RayPre& world_set(RayPre& r, f3 o, f3 d) {
     return r;
 }
 __device__ __forceinline__ f3 world_o(const WorldRaySlot& w) { return mk(w.p[0], w.p[128], w.p[256]); }
-__device__ __forceinline__ f3 world_d(const WorldRaySlot& w) { return mk(w.p[384], w.p[512], w.p[640]); }
+__device__ __forceinline__ f3 world_d(const WorldRaySlot& w) {
+    const float4 d = *w.ray;
+    return mk(d.x, d.y, d.z);
+}
 __device__ __forceinline__ RayPre world_pre(const WorldRaySlot& w) {
-    RayPre r;
-    r.o = world_o(w);
-    r.d[0] = w.p[384]; r.d[1] = w.p[512]; r.d[2] = w.p[640];
-    r.kx = __float_as_int(w.p[768]); r.ky = __float_as_int(w.p[896]); r.kz = __float_as_int(w.p[1024]);
-    r.Sx = w.p[1152]; r.Sy = w.p[1280]; r.Sz = w.p[1408];
-    r.invd[0] = w.p[1536]; r.invd[1] = w.p[1664]; r.invd[2] = w.p[1792];
-    r.near = __float_as_uint(w.p[1920]);
+    RayPre r = ray_pre(world_o(w), world_d(w));  // the triangle-test half, where the caller uses it
+    r.invd[0] = w.p[384]; r.invd[1] = w.p[512]; r.invd[2] = w.p[640];
+    r.near = (r.invd[0] < 0.f ? 1u : 0u) | (r.invd[1] < 0.f ? 2u : 0u) | (r.invd[2] < 0.f ? 4u : 0u);
     return r;
 }
 __device__ __forceinline__ RayPre world_set(WorldRaySlot& w, f3 o, f3 d) {
     const RayPre r = ray_pre(o, d);
     w.p[0] = r.o.x; w.p[128] = r.o.y; w.p[256] = r.o.z;
-    w.p[384] = r.d[0]; w.p[512] = r.d[1]; w.p[640] = r.d[2];
-    w.p[768] = __int_as_float(r.kx); w.p[896] = __int_as_float(r.ky); w.p[1024] = __int_as_float(r.kz);
-    w.p[1152] = r.Sx; w.p[1280] = r.Sy; w.p[1408] = r.Sz;
-    w.p[1536] = r.invd[0]; w.p[1664] = r.invd[1]; w.p[1792] = r.invd[2];
-    w.p[1920] = __uint_as_float(r.near);
+    w.p[384] = r.invd[0]; w.p[512] = r.invd[1]; w.p[640] = r.invd[2];
     return r;
 }
 
@@ -567,28 +570,29 @@ __device__ __forceinline__ const RayPre& cur_ray(const Trav& t, const RW& rw) {
 // TLAS group on the stack, moves the ray into object space and walks the
 // BLAS above the saved stack height; once that part of the stack is empty
 // the world ray is restored.  Returns false when the walk is over.
-template <class Stack, class RW>
+template <class Stack, class RW, class Status>
 __device__ __forceinline__ bool two_level_settle(const SceneDev& S, const RW& rw, Trav& t, Stack stk,
-                                                 uint32_t* status) {
+                                                 Status status) {
     for (;;) {
         if (!t.level && t.inst_bits) {
             if (t.g_bits & 0xff000000u) {
-                if (t.sp >= S.stack_cap) { atomicOr(status, HY_STATUS_STACK_OVERFLOW); return false; }
+                if (t.sp >= S.stack_cap) { raise_status(status, HY_STATUS_STACK_OVERFLOW); return false; }
                 stack_put(stk, t.sp, make_uint2(t.g_base, t.g_bits));
                 t.sp++;
             }
             const uint32_t b = __ffs(t.inst_bits) - 1;
             t.inst_bits &= t.inst_bits - 1u;
             const uint32_t rec = t.inst_base + b;
-            if (rec >= S.num_tris) { atomicOr(status, HY_STATUS_BAD_INDEX); return false; }
+            if (rec >= S.num_tris) { raise_status(status, HY_STATUS_BAD_INDEX); return false; }
             const uint32_t iid = __float_as_uint(__ldg(&S.tris[(size_t)rec * 3].w));
-            if (iid >= S.num_inst) { atomicOr(status, HY_STATUS_BAD_INDEX); return false; }
+            if (iid >= S.num_inst) { raise_status(status, HY_STATUS_BAD_INDEX); return false; }
             const float4* I = S.inst + (size_t)iid * 4;
             const float4 r0 = __ldg(I), r1 = __ldg(I + 1), r2 = __ldg(I + 2), m = __ldg(I + 3);
             t.cur = ray_pre(xform_point(r0, r1, r2, world_o(rw)), xform_dir(r0, r1, r2, world_d(rw)));
             t.level = true;
             t.sp_base = t.sp;
             t.id_off = __float_as_uint(m.y);
+            t.inst = iid;
             t.g_base = __float_as_uint(m.x);
             t.g_bits = 1u << 24;  // virtual group holding the BLAS root
             return true;
@@ -616,13 +620,10 @@ __device__ __forceinline__ bool two_level_settle(const SceneDev& S, const RW& rw
 // the same node visits and triangle tests, in the same order, as a walk that
 // tests each node's triangles at once.
 // TWO: the two-level structure (r is the world ray; t.cur the current one).
-// top / ntop: the structure's first ntop nodes (its top levels, BFS order)
-// staged in shared memory by the caller's block.
-template <bool ANY, bool COUNT, bool TWO = false, class Stack = uint2*, class RW = RayPre>
+template <bool ANY, bool COUNT, bool TWO = false, class Stack = uint2*, class RW = RayPre, class Status = uint32_t*>
 __device__ __forceinline__ bool trav_node(const SceneDev& S, const RW& rw, float tmin, Trav& t, Stack stk,
-                                          uint32_t& nodes_ctr, uint32_t* status, const uint4* top = nullptr,
-                                          uint32_t ntop = 0) {
-    if (++t.iters > S.max_iters) { atomicOr(status, HY_STATUS_TIMEOUT); return true; }
+                                          uint32_t& nodes_ctr, Status status) {
+    if (++t.iters > S.max_iters) { raise_status(status, HY_STATUS_TIMEOUT); return true; }
     if (TWO) {
         if (!two_level_settle(S, rw, t, stk, status)) return true;
     } else if ((t.g_bits & 0xff000000u) == 0) {
@@ -639,19 +640,13 @@ __device__ __forceinline__ bool trav_node(const SceneDev& S, const RW& rw, float
     const uint32_t sl = rb ^ ord;
     const uint32_t idx = t.g_base + __popc(t.g_bits & 0xffu & ((1u << sl) - 1u));
     if (t.g_bits & 0xff000000u) {
-        if (t.sp >= S.stack_cap) { atomicOr(status, HY_STATUS_STACK_OVERFLOW); return true; }
+        if (t.sp >= S.stack_cap) { raise_status(status, HY_STATUS_STACK_OVERFLOW); return true; }
         stack_put(stk, t.sp, make_uint2(t.g_base, t.g_bits));
         t.sp++;
     }
-    if (idx >= S.num_nodes) { atomicOr(status, HY_STATUS_BAD_INDEX); return true; }
-    uint4 q0, q1, q2, q3, q4;
-    if (idx < ntop) {
-        const uint4* np = top + (size_t)idx * 5;
-        q0 = np[0]; q1 = np[1]; q2 = np[2]; q3 = np[3]; q4 = np[4];
-    } else {
-        const uint4* np = S.nodes[idx].q;
-        q0 = __ldg(np + 0); q1 = __ldg(np + 1); q2 = __ldg(np + 2); q3 = __ldg(np + 3); q4 = __ldg(np + 4);
-    }
+    if (idx >= S.num_nodes) { raise_status(status, HY_STATUS_BAD_INDEX); return true; }
+    const uint4* np = S.nodes[idx].q;
+    const uint4 q0 = __ldg(np + 0), q1 = __ldg(np + 1), q2 = __ldg(np + 2), q3 = __ldg(np + 3), q4 = __ldg(np + 4);
     if (COUNT) nodes_ctr++;
     float adj[3], org[3];
     const float p[3] = {__uint_as_float(q0.x), __uint_as_float(q0.y), __uint_as_float(q0.z)};
@@ -764,9 +759,8 @@ __device__ __forceinline__ bool trav_tri(const SceneDev& S, const RW& rw, float 
 // Returns true when the ray is finished: t.h holds the hit, or id HY_NO_HIT.
 template <bool ANY, bool COUNT, bool TWO = false, class Stack = uint2*, class RW = RayPre>
 __device__ __forceinline__ bool trav_step(const SceneDev& S, const RW& rw, float tmin, Trav& t, Stack stk,
-                                          uint32_t& nodes_ctr, uint32_t& tris_ctr, uint32_t* status,
-                                          const uint4* top = nullptr, uint32_t ntop = 0) {
-    if (trav_node<ANY, COUNT, TWO>(S, rw, tmin, t, stk, nodes_ctr, status, top, ntop)) return true;
+                                          uint32_t& nodes_ctr, uint32_t& tris_ctr, uint32_t* status) {
+    if (trav_node<ANY, COUNT, TWO>(S, rw, tmin, t, stk, nodes_ctr, status)) return true;
     while (t.pend_bits)
         if (trav_tri<ANY, COUNT, TWO>(S, rw, tmin, t, tris_ctr, status)) return true;
     return false;

@@ -5,6 +5,8 @@
 // the hybrid pass.  One lane per pixel; persistent warps pull 8x4 tiles.
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "hy_shade.cuh"
 #include "hy_stream.cuh"
 
@@ -270,7 +272,8 @@ __global__ void __launch_bounds__(128) k_pathtrace(const SceneDev S, const PtPar
 // in the same order, so the image equals k_pathtrace's.
 template <bool COUNT, bool TWO, int MINB>
 __global__ void __launch_bounds__(128, MINB) k_pathtrace_stream(const SceneDev S, const PtParams T) {
-    __shared__ StreamSlots sm;
+    __shared__ StreamSlotsT<4, TWO> sm;
+    __shared__ float s_world[TWO ? 6 * 128 : 1];  // two-level: WorldRaySlot words
     const PassParams& P = T.P;
     LaneStats ls;
     const uint32_t lane = threadIdx.x & 31, wb = threadIdx.x & ~31u;
@@ -279,7 +282,11 @@ __global__ void __launch_bounds__(128, MINB) k_pathtrace_stream(const SceneDev S
     const float spp = (float)P.spp;
     uint2 stk[kStackMax];
     Trav t;
-    RayPre r;
+    std::conditional_t<TWO, WorldRaySlot, RayPre> r{};
+    if constexpr (TWO) {
+        r.p = s_world + threadIdx.x;
+        r.ray = &sm.scratch[threadIdx.x >> 5].walk.ray[lane];
+    }
     uint32_t nn = 0, nt = 0;
     for (;;) {
         uint32_t t0 = 0;
@@ -325,7 +332,7 @@ __global__ void __launch_bounds__(128, MINB) k_pathtrace_stream(const SceneDev S
                                    traced ? g.dist : 0.f, !traced || reference ? seed : lcg_jump(seed, 2u * rays_before));
                     // closesthit.rchit: origin worldPos + 0.01 dir, tmax distance + 1
                     if (__ballot_sync(0xffffffffu, traced) != 0)
-                        stream_light<COUNT, TWO>(S, P, sm, nrays, lt.radius, 1e-2f, stk, t, r, ls, nn, nt, nullptr, 0);
+                        stream_light<COUNT, TWO>(S, P, sm, nrays, lt.radius, 1e-2f, stk, t, r, ls, nn, nt);
                     if (hit) {
                         float sf = 0.f;
                         if (g.NdotL > 0.f) {

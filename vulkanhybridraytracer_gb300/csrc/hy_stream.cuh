@@ -3,10 +3,11 @@
 // publishes one pixel's shadow-ray inputs (position, distance, sampleDisk's
 // frame, the RNG state of the pixel-light's first sample) in shared memory;
 // the warp then traces the 32 x n_rays samples as items q (sample q % n_rays of
-// pixel q / n_rays), claimed in order from a per-warp counter by whichever
-// lanes are free, each lane walking its rays with several node visits per
-// scheduling round and without waiting for the others; unoccluded samples are
-// counted per pixel with shared-memory atomics.
+// pixel q / n_rays), taken in order by whichever lanes are free, each lane
+// walking its rays with several node visits per scheduling round and without
+// waiting for the others' rays to end; the triangles a round reaches are tested
+// by the whole warp together; unoccluded samples are counted per pixel with
+// shared-memory atomics.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -25,31 +26,37 @@ namespace hy {
 // chunks of SORT items per warp and light.
 // The size matters beyond occupancy: shared memory and L1 share each SM's
 // 256 KB, and the driver carves shared memory in steps (..., 100, 132, 164,
-// 196 KB).  At 4 warps per block and 8 blocks per SM this layout (15.4 KB, + 1
-// KB the driver keeps per block) takes the 132 KB step and leaves the kernel
-// 124 KB of L1 for the nodes, triangles and traversal stacks it re-reads
-// (the same slots with a separate count array and 73 top nodes staged per
-// block took the 196 KB step: 1080p shadow kernel 22.5 ms against 22.2 ms with
-// 92 KB of L1 and no staging).
+// 196 KB).  The sort's scratch and the walk's are used in turn and overlap, so
+// at 4 warps per block and 8 blocks per SM this layout (15.3 KB, + 1 KB the
+// driver keeps per block) takes the 132 KB step and leaves the kernel 124 KB of
+// L1 for the nodes, triangles and traversal stacks it re-reads; the two-level
+// kernel (instance ids per pair, 3 KB of world rays) takes the 164 KB step.
 constexpr uint32_t kSortItems = 512, kSortBuckets = 64;
-template <int NW, uint32_t SORT = kSortItems>  // warps per block, items sorted together
+constexpr uint32_t kPairs = 64;  // (ray, triangle) pairs a warp collects between two test phases
+template <int NW, bool TWO = false, uint32_t SORT = kSortItems>  // warps per block, items sorted together
 struct StreamSlotsT {
     static constexpr uint32_t kSort = SORT;
-    // the sort keys of a light's items: in shared memory up to 4 warps per block,
-    // in a chain of registers beyond (8-warp batch blocks: 30 KB instead of 34 KB,
-    // under the 132 KB shared-memory step at 4 blocks per SM)
-    static constexpr bool kKeysShared = NW <= 4;
     float4 pos[NW * 32];
     float4 PL[NW * 32];
     float4 T[NW * 32];
     float4 B[NW * 32];
-    uint32_t next[NW];  // per warp: the next unclaimed item of the current light
-    // per warp: the traced items of the light ordered by their disk sample, the
-    // sample's cell per item (kKeysShared) and the cell counts / cursors of the
-    // counting sort
-    uint16_t order[NW][SORT];
-    uint8_t key[kKeysShared ? NW : 1][kKeysShared ? SORT : 1];
-    uint32_t bucket[NW][kSortBuckets];
+    uint16_t order[NW][SORT];  // per warp: the traced items of the light ordered by their disk sample
+    uint32_t npairs[NW];       // per warp: pairs collected (may count past kPairs: those wait on their lanes)
+    union Scratch {
+        // the sort: the sample's cell per item, the cell counts / cursors
+        struct {
+            uint8_t key[SORT];
+            uint32_t bucket[kSortBuckets];
+        } sort;
+        // the walk: each lane's ray (direction, tmax) and the pairs waiting for their test
+        struct {
+            float4 ray[32];
+            uint32_t rec[kPairs];
+            uint32_t inst[TWO ? kPairs : 1];
+            uint8_t owner[kPairs];
+        } walk;
+    };
+    alignas(16) Scratch scratch[NW];
 };
 using StreamSlots = StreamSlotsT<4>;
 
@@ -76,7 +83,65 @@ __device__ __forceinline__ void stream_publish(Slots& sm, bool traced, f3 positi
         sm.T[i].w = __uint_as_float(kNotTraced);
         sm.B[i].w = 0.f;
     }
-    if ((i & 31) == 0) sm.next[i >> 5] = 0;
+}
+
+// The triangles of the leaf slots a lane's last node visit hit, put into the
+// warp's pair list; what does not fit stays in t.pend_bits.
+template <bool TWO, class Slots>
+__device__ __forceinline__ void pairs_push(Slots& sm, Trav& t) {
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    auto& w = sm.scratch[warp].walk;
+    uint32_t at = atomicAdd(&sm.npairs[warp], (uint32_t)__popc(t.pend_bits));
+    while (t.pend_bits && at < kPairs) {
+        const uint32_t b = __ffs(t.pend_bits) - 1;
+        t.pend_bits &= t.pend_bits - 1u;
+        w.rec[at] = t.pend_base + b;
+        w.owner[at] = (uint8_t)lane;
+        if (TWO) w.inst[at] = t.inst;
+        at++;
+    }
+}
+
+// Tests the warp's pairs, one per lane: the lane takes the ray of the pair's
+// owner (origin by shuffle, direction and tmax from the owner's slot; two-level:
+// moved into the pair's instance) and sets it up for the test as the owner would
+// have.  Returns the mask of owners with a hit.  All lanes call it, np uniform.
+template <bool TWO, class Slots, class RW>
+__device__ __forceinline__ uint32_t pairs_test(const SceneDev& S, Slots& sm, uint32_t np, const RW& r, float tmin,
+                                               uint32_t* status) {
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const auto& w = sm.scratch[warp].walk;
+    uint32_t hits = 0;
+    for (uint32_t b = 0; b < np; b += 32) {
+        const uint32_t i = b + lane;
+        const bool valid = i < np;
+        const uint32_t owner = valid ? (uint32_t)w.owner[i] : lane;
+        f3 o;
+        if constexpr (TWO) {
+            const int d = (int)owner - (int)lane;
+            o = mk(r.p[d], r.p[d + 128], r.p[d + 256]);
+        } else {
+            o = mk(__shfl_sync(0xffffffffu, r.o.x, owner), __shfl_sync(0xffffffffu, r.o.y, owner),
+                   __shfl_sync(0xffffffffu, r.o.z, owner));
+        }
+        if (valid) {
+            const uint32_t rec = w.rec[i];
+            if (rec >= S.num_tris) { atomicOr(status, HY_STATUS_BAD_INDEX); continue; }
+            const float4 ray = w.ray[owner];
+            f3 dir = mk(ray.x, ray.y, ray.z);
+            if constexpr (TWO) {
+                const float4* I = S.inst + (size_t)w.inst[i] * 4;
+                const float4 r0 = __ldg(I), r1 = __ldg(I + 1), r2 = __ldg(I + 2);
+                o = xform_point(r0, r1, r2, o);
+                dir = xform_dir(r0, r1, r2, dir);
+            }
+            const float4* tp = S.tris + (size_t)rec * 3;
+            float tt, b1, b2;
+            if (tri_test(ray_pre(o, dir), __ldg(tp), __ldg(tp + 1), __ldg(tp + 2), tmin, ray.w, tt, b1, b2))
+                hits |= 1u << owner;
+        }
+    }
+    return __reduce_or_sync(0xffffffffu, hits);
 }
 
 // The warp's items of one light (every lane calls it, after all lanes have
@@ -84,13 +149,30 @@ __device__ __forceinline__ void stream_publish(Slots& sm, bool traced, f3 positi
 // steps (sampleDisk's two draws per sample), its ray from position +
 // offset * dir to distance + 1.  On return unocc_count holds each pixel's
 // unoccluded samples.
+//
+// A round is: idle lanes take the light's next items; up to P.inner node visits
+// per lane; the triangles those visits reached, tested together.  A lane does
+// not test its triangles where it finds them: it puts (ray, triangle) pairs into
+// the warp's list and walks on, and at the end of the round the warp's lanes take
+// one pair each.  On the 1080p frame a node visit of the warp reaches 2.5
+// triangles, on 2.5 lanes: tested at once they took as many warp instructions
+// as a third of the whole kernel; collected over a round they fill the lanes
+// (4.85 -> 4.27 G warp instructions on the 960x540 frame, 15.5 -> 20.2 lanes each;
+// 1080p shadow kernel 20.1 -> 17.9 ms, 1277x719 two-level 16.3 -> 13.0 ms).
+// A lane whose ray has already found its occluder walks on until the round ends,
+// where it would have waited for the round anyway.  The outcome of a ray does not
+// change: any-hit walks visit the same nodes whatever was hit before, so the
+// triangles tested are those of the plain walk up to its first hit and a few
+// more of a ray that is known to be occluded by then.  A limit that runs out
+// (node visits, stack) is reported only if none of the ray's waiting pairs hit.
+// COUNT: the plain walk, each visit's triangles tested at once, so the counts are
+// those of each ray's walk up to its first hit.
 template <bool COUNT, bool TWO, class Stack, class Slots, class RW>
 __device__ __forceinline__ void stream_light(const SceneDev& S, const PassParams& P, Slots& sm, uint32_t nrays,
                                              float radius, float offset, Stack stk, Trav& t, RW& r,
-                                             LaneStats& ls, uint32_t& nn, uint32_t& nt, const uint4* top,
-                                             uint32_t ntop) {
+                                             LaneStats& ls, uint32_t& nn, uint32_t& nt) {
     const uint32_t lane = threadIdx.x & 31, wb = threadIdx.x & ~31u, warp = threadIdx.x >> 5;
-    uint32_t* next = &sm.next[warp];
+    const uint32_t lt_mask = (1u << lane) - 1u;
     const uint32_t all = 32u * nrays;
     __syncwarp();
     // the light's items in chunks of Slots::kSort (one chunk unless spp > 16)
@@ -105,23 +187,15 @@ __device__ __forceinline__ void stream_light(const SceneDev& S, const PassParams
         //      not change: only which lane traces which ray, and when ----
         const bool sorted = nrays > 1;
         if (sorted) {
-            uint32_t* bk = sm.bucket[warp];
+            uint32_t* bk = sm.scratch[warp].sort.bucket;
+            uint8_t* keys = sm.scratch[warp].sort.key;
             bk[lane] = 0;
             bk[lane + 32] = 0;
             __syncwarp();
-            // each lane's item keys (items lane + 32 i, one byte each) go to shared
-            // memory or through a shift chain of registers: after the kSort / 32
-            // steps item i's key is byte i
-            constexpr uint32_t kSteps = Slots::kSort / 32, kWords = kSteps / 4;
-            static_assert(kSteps % 4 == 0, "whole key words");
-            uint32_t keys[kWords];
-#pragma unroll
-            for (uint32_t w = 0; w < kWords; w++) keys[w] = 0;
-            for (uint32_t i = 0; i < kSteps; i++) {
-                const uint32_t j = lane + 32u * i;
+            for (uint32_t j = lane; j < cn; j += 32) {
                 uint32_t key = 0xffu;
-                const uint32_t q = c0 + j, pi = j < cn ? q / nrays : 0u, k = q - pi * nrays;
-                if (j < cn && __float_as_uint(sm.T[wb + pi].w) != kNotTraced) {
+                const uint32_t q = c0 + j, pi = q / nrays, k = q - pi * nrays;
+                if (__float_as_uint(sm.T[wb + pi].w) != kNotTraced) {
                     uint32_t st = lcg_jump_even(__float_as_uint(sm.PL[wb + pi].w), k);
                     const float r1 = rnd(st), r2 = rnd(st);
                     // the disk point in units of the radius (approximate: it only orders the items)
@@ -134,19 +208,13 @@ __device__ __forceinline__ void stream_light(const SceneDev& S, const PassParams
                           ((iy & 4u) << 3);
                     atomicAdd(&bk[key], 1u);
                 }
-                if constexpr (Slots::kKeysShared) {
-                    if (j < cn) sm.key[warp][j] = (uint8_t)key;
-                } else {
-#pragma unroll
-                    for (uint32_t w = 0; w + 1 < kWords; w++) keys[w] = (keys[w] >> 8) | (keys[w + 1] << 24);
-                    keys[kWords - 1] = (keys[kWords - 1] >> 8) | (key << 24);
-                }
+                keys[j] = (uint8_t)key;
             }
             __syncwarp();
             // exclusive scan of the 64 counts, two per lane
             const uint32_t cnt0 = bk[2 * lane], cnt1 = bk[2 * lane + 1], c = cnt0 + cnt1;
             uint32_t incl = c;
-    #pragma unroll
+#pragma unroll
             for (int d = 1; d < 32; d <<= 1) {
                 const uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
                 if (lane >= (uint32_t)d) incl += y;
@@ -156,66 +224,86 @@ __device__ __forceinline__ void stream_light(const SceneDev& S, const PassParams
             bk[2 * lane] = incl - c;
             bk[2 * lane + 1] = incl - c + cnt0;
             __syncwarp();
-            for (uint32_t i = 0; i < kSteps; i++) {
-                const uint32_t j = lane + 32u * i;
-                uint32_t key;
-                if constexpr (Slots::kKeysShared) {
-                    if (j >= cn) break;
-                    key = sm.key[warp][j];
-                } else {
-                    key = keys[0] & 0xffu;
-#pragma unroll
-                    for (uint32_t w = 0; w + 1 < kWords; w++) keys[w] = (keys[w] >> 8) | (keys[w + 1] << 24);
-                    keys[kWords - 1] >>= 8;
-                    if (j >= cn) continue;
-                }
+            for (uint32_t j = lane; j < cn; j += 32) {
+                const uint32_t key = keys[j];
                 if (key != 0xffu) sm.order[warp][atomicAdd(&bk[key], 1u)] = (uint16_t)j;
             }
         }
-        if (lane == 0) *next = 0;
+        if (lane == 0) sm.npairs[warp] = 0;
         __syncwarp();
-        bool live = false, more = true;
-        uint32_t cur = 0;
+        bool live = false;
+        uint32_t cur = 0, head = 0;  // head: the first unclaimed item (the same on every lane)
         for (;;) {
-            // ---- this lane's next item of a traced pixel, claimed from the warp's
-            //      counter: items go to whichever lanes are free, in order, so the
-            //      warp's work stays balanced until the light's last items ----
-            while (!live && more) {
-                // one shared atomic per group of lanes claiming together, lane order kept
-                const uint32_t m = __activemask(), leader = __ffs(m) - 1;
-                uint32_t base = 0;
-                if (lane == leader) base = atomicAdd(next, (uint32_t)__popc(m));
-                base = __shfl_sync(m, base, leader);
-                uint32_t q = base + (uint32_t)__popc(m & ((1u << lane) - 1u));
-                if (q >= total) { more = false; break; }
-                q = c0 + (sorted ? (uint32_t)sm.order[warp][q] : q);
-                const uint32_t pi = q / nrays, k = q - pi * nrays;
-                const float4 tp = sm.T[wb + pi];
-                if (__float_as_uint(tp.w) == kNotTraced) continue;
-                const float4 pp = sm.pos[wb + pi], pl = sm.PL[wb + pi], bp = sm.B[wb + pi];
-                const f3 pos = mk(pp.x, pp.y, pp.z);
-                const DiskFrame d{mk(tp.x, tp.y, tp.z), mk(bp.x, bp.y, bp.z), mk(pl.x, pl.y, pl.z)};
-                uint32_t st = lcg_jump_even(__float_as_uint(pl.w), k);
-                const f3 dir = sampleDisk(radius, pos, d, st);
-                trav_init(t, world_set(r, add_rn(pos, scale_rn(dir, offset)), dir), __fadd_rn(pp.w, 1.0f));
-                cur = pi;
-                live = true;
-                ls.shadow++;
+            // ---- idle lanes take the next items, in order ----
+            const uint32_t idle = __ballot_sync(0xffffffffu, !live);
+            if (head < total) {
+                const uint32_t at = head + (uint32_t)__popc(idle & lt_mask);
+                head += (uint32_t)__popc(idle);
+                if (!live && at < total) {
+                    const uint32_t q = c0 + (sorted ? (uint32_t)sm.order[warp][at] : at);
+                    const uint32_t pi = q / nrays, k = q - pi * nrays;
+                    const float4 tp = sm.T[wb + pi];
+                    if (__float_as_uint(tp.w) != kNotTraced) {
+                        const float4 pp = sm.pos[wb + pi], pl = sm.PL[wb + pi], bp = sm.B[wb + pi];
+                        const f3 pos = mk(pp.x, pp.y, pp.z);
+                        const DiskFrame d{mk(tp.x, tp.y, tp.z), mk(bp.x, bp.y, bp.z), mk(pl.x, pl.y, pl.z)};
+                        uint32_t st = lcg_jump_even(__float_as_uint(pl.w), k);
+                        const f3 dir = sampleDisk(radius, pos, d, st);
+                        const float tmax = __fadd_rn(pp.w, 1.0f);
+                        sm.scratch[warp].walk.ray[lane] = make_float4(dir.x, dir.y, dir.z, tmax);
+                        trav_init(t, world_set(r, add_rn(pos, scale_rn(dir, offset)), dir), tmax);
+                        cur = pi;
+                        live = true;
+                        ls.shadow++;
+                    }
+                }
+            } else if (idle == 0xffffffffu) {
+                break;
             }
-            // ---- up to P.inner node visits, each with its leaf triangles (testing
-            //      the triangles of many lanes together instead, once enough lanes
-            //      have some, measured slower: 2,190 against 2,899 Mrays/s at 1080p,
-            //      the lanes waiting on triangles idle through the node visits) ----
+            // ---- up to P.inner node visits ----
+            bool over = false, occluded = false;
+            uint32_t limits = 0;
             if (live) {
                 for (uint32_t it = 0, ni = max(P.inner, 1u); it < ni; it++) {
-                    if (trav_step<true, COUNT, TWO>(S, r, 0.001f, t, stk, nn, nt, P.status, top, ntop)) {
-                        live = false;
-                        if (t.h.id == HY_NO_HIT) atomicAdd(unocc_count(sm, wb + cur), 1u);
-                        break;
+                    if constexpr (COUNT) {
+                        if (trav_step<true, true, TWO>(S, r, 0.001f, t, stk, nn, nt, P.status)) {
+                            over = true;
+                            occluded = t.h.id != HY_NO_HIT;
+                            break;
+                        }
+                    } else {
+                        if (trav_node<true, false, TWO>(S, r, 0.001f, t, stk, nn, DeferredStatus{limits})) {
+                            over = true;
+                            break;
+                        }
+                        if (t.pend_bits) {
+                            pairs_push<TWO>(sm, t);
+                            if (t.pend_bits) break;  // the list is full: the rest after the test below
+                        }
                     }
                 }
             }
-            if (__ballot_sync(0xffffffffu, live || more) == 0) break;
+            // ---- the round's triangles ----
+            if constexpr (!COUNT) {
+                for (;;) {
+                    __syncwarp();
+                    const uint32_t np = min(sm.npairs[warp], kPairs);
+                    if (np == 0) break;
+                    const uint32_t hits = pairs_test<TWO>(S, sm, np, r, 0.001f, P.status);
+                    if (lane == 0) sm.npairs[warp] = 0;
+                    if ((hits >> lane) & 1u) { occluded = true; t.pend_bits = 0; }
+                    __syncwarp();
+                    if (__ballot_sync(0xffffffffu, live && t.pend_bits != 0) == 0) break;
+                    if (live && t.pend_bits) pairs_push<TWO>(sm, t);
+                }
+            }
+            if (live && (over || occluded)) {
+                live = false;
+                if (!occluded) {
+                    if (limits) atomicOr(P.status, limits);
+                    atomicAdd(unocc_count(sm, wb + cur), 1u);
+                }
+            }
         }
         __syncwarp();
     }
@@ -255,8 +343,7 @@ __device__ __forceinline__ void shadow_finalize(const PassParams& P, const Shado
 template <bool COUNT, bool TWO, int ACC, class Stack, class Slots, class RW>
 __device__ __forceinline__ void stream_tile(const SceneDev& S, const PassParams& P, uint32_t tile, bool reference,
                                             bool accum, Slots& sm, Stack stk, Trav& t, RW& r,
-                                            ShadowLane& s, LaneStats& ls, uint32_t& nn, uint32_t& nt,
-                                            const uint4* top, uint32_t ntop) {
+                                            ShadowLane& s, LaneStats& ls, uint32_t& nn, uint32_t& nt) {
     const uint32_t lane = threadIdx.x & 31, wb = threadIdx.x & ~31u;
     const size_t plane = (size_t)P.W * P.H;
     const uint32_t spp = P.spp, nrays = reference ? 1u : spp;
@@ -298,7 +385,7 @@ __device__ __forceinline__ void stream_tile(const SceneDev& S, const PassParams&
         }
         if (__ballot_sync(0xffffffffu, traced) != 0) {
             // shadowRaygen.rgen:78: origin position + 0.1 dir, tmax distance + 1
-            stream_light<COUNT, TWO>(S, P, sm, nrays, S.lights[l].radius, 1e-1f, stk, t, r, ls, nn, nt, top, ntop);
+            stream_light<COUNT, TWO>(S, P, sm, nrays, S.lights[l].radius, 1e-1f, stk, t, r, ls, nn, nt);
             if (traced) {
                 const uint32_t unocc = *unocc_count(sm, wb + lane);
                 finalize(reference ? (float)unocc : __fdiv_rn((float)unocc, (float)spp));

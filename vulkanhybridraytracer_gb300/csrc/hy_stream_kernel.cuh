@@ -35,19 +35,19 @@ namespace hy {
 // ---------------------------------------------------------------------------------
 template <bool COUNT, bool ACCUM, int MINB, bool TWO = false, bool SHORT = false>
 __global__ void __launch_bounds__(128, MINB) k_shadow_stream(const SceneDev S, const PassParams P) {
-    __shared__ StreamSlots sm;
+    __shared__ StreamSlotsT<4, TWO> sm;
     __shared__ uint2 s_stack[SHORT ? kShortStack * 128 : 1];
-    // two-level: each lane's world ray set-up (WorldRaySlot, 64 B a lane): 8
-    // blocks at 23.6 KB stay on the 196 KB shared-memory step (the 68-byte
-    // padded layout of the same data took 24.1 KB and the 228 KB step)
-    __shared__ float s_world[TWO ? 16 * 128 : 1];
+    __shared__ float s_world[TWO ? 6 * 128 : 1];  // two-level: WorldRaySlot words
     LaneStats ls;
     const uint32_t lane = threadIdx.x & 31;
     uint2 stk[kStackMax];
     ShadowLane s;
     Trav t;
     std::conditional_t<TWO, WorldRaySlot, RayPre> r{};
-    if constexpr (TWO) r.p = s_world + threadIdx.x;
+    if constexpr (TWO) {
+        r.p = s_world + threadIdx.x;
+        r.ray = &sm.scratch[threadIdx.x >> 5].walk.ray[lane];
+    }
     uint32_t chunk_cur = 0, chunk_end = 0, nn = 0, nt = 0;
     for (;;) {
         if (chunk_cur == chunk_end) {
@@ -60,11 +60,10 @@ __global__ void __launch_bounds__(128, MINB) k_shadow_stream(const SceneDev S, c
         }
         if (SHORT)
             stream_tile<COUNT, TWO, ACCUM ? 1 : 0>(S, P, chunk_cur++, P.rng_mode == HY_RNG_REFERENCE, ACCUM, sm,
-                                                   SplitStack{s_stack + threadIdx.x, stk}, t, r, s, ls, nn, nt, nullptr,
-                                                   0u);
+                                                   SplitStack{s_stack + threadIdx.x, stk}, t, r, s, ls, nn, nt);
         else
             stream_tile<COUNT, TWO, ACCUM ? 1 : 0>(S, P, chunk_cur++, P.rng_mode == HY_RNG_REFERENCE, ACCUM, sm, stk, t,
-                                                   r, s, ls, nn, nt, nullptr, 0u);
+                                                   r, s, ls, nn, nt);
     }
     if (COUNT) { ls.nodes += nn; ls.tris += nt; }
     flush_stats(ls, P.stats);
