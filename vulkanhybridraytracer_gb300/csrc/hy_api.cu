@@ -690,6 +690,25 @@ int hy_bvh_refit(HyCtx* c, const float* xf, uint32_t nx) {
     return bvh_refit_impl(c);
 }
 
+// nodes [n] as the documented 20 words: the device keeps each slot's lo and hi
+// plane bytes side by side (hy_device.cuh), the caller gets them per plane
+static int download_nodes(const HyCtx* c, uint32_t* out) {
+    const size_t n = c->n_bvh8;
+    HY_CUDA_TRY(cudaMemcpy(out, c->nodes.p, n * sizeof(Node8), cudaMemcpyDeviceToHost));
+    for (size_t i = 0; i < n; i++) {
+        uint32_t* w = out + i * 20 + 8;
+        uint32_t planes[12] = {};  // lo x, y, z, then hi x, y, z, two words each
+        for (int a = 0; a < 3; a++)
+            for (int sl = 0; sl < 8; sl++) {
+                const uint32_t pair = w[a * 4 + (sl >> 1)] >> ((sl & 1) * 16);
+                planes[a * 2 + (sl >> 2)] |= (pair & 0xffu) << ((sl & 3) * 8);
+                planes[6 + a * 2 + (sl >> 2)] |= ((pair >> 8) & 0xffu) << ((sl & 3) * 8);
+            }
+        std::memcpy(w, planes, sizeof(planes));
+    }
+    return HY_OK;
+}
+
 int hy_bvh_download(HyCtx* c, uint32_t* morton, uint32_t* order, uint32_t* bvh2, uint32_t* bvh8, float* tris) {
     if (!c) return HY_ERR_INVALID_ARG;
     if (!c->bvh_ok) return HY_ERR_NOT_READY;
@@ -698,14 +717,16 @@ int hy_bvh_download(HyCtx* c, uint32_t* morton, uint32_t* order, uint32_t* bvh2,
     if (c->two_level && (morton || order || bvh2)) return HY_ERR_INVALID_ARG;  // nodes and records only
     HY_CUDA_TRY(cudaStreamSynchronize(c->stream));
     if (c->two_level) {
-        if (bvh8) HY_CUDA_TRY(cudaMemcpy(bvh8, c->nodes.p, (size_t)c->n_bvh8 * 80, cudaMemcpyDeviceToHost));
+        int rc;
+        if (bvh8 && (rc = download_nodes(c, bvh8))) return rc;
         if (tris) HY_CUDA_TRY(cudaMemcpy(tris, c->tris.p, (size_t)c->n_records * 48, cudaMemcpyDeviceToHost));
         return HY_OK;
     }
     if (morton) HY_CUDA_TRY(cudaMemcpy(morton, c->keys[0].p, n * 4, cudaMemcpyDeviceToHost));
     if (order) HY_CUDA_TRY(cudaMemcpy(order, c->vals[0].p, n * 4, cudaMemcpyDeviceToHost));
     if (bvh2 && n > 1) HY_CUDA_TRY(cudaMemcpy(bvh2, c->bvh2.p, (n - 1) * 40, cudaMemcpyDeviceToHost));
-    if (bvh8) HY_CUDA_TRY(cudaMemcpy(bvh8, c->nodes.p, (size_t)c->n_bvh8 * 80, cudaMemcpyDeviceToHost));
+    int rc;
+    if (bvh8 && (rc = download_nodes(c, bvh8))) return rc;
     if (tris) HY_CUDA_TRY(cudaMemcpy(tris, c->tris.p, n * 48, cudaMemcpyDeviceToHost));
     return HY_OK;
 }

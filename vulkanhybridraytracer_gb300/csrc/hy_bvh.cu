@@ -532,7 +532,7 @@ __global__ void k_collapse_plan(const uint32_t* __restrict__ lvl, uint32_t m, co
 // quantised outwards: floor((lo - p)_rd / 2^e), ceil((hi - p)_ru / 2^e).
 __device__ __forceinline__ void quantize_node(const Ref& nb, const uint32_t* slots, const uint32_t* bvh2,
                                               const uint32_t* order, const float* tribox, uint32_t& e3,
-                                              uint32_t qlo[3][2], uint32_t qhi[3][2]) {
+                                              uint32_t q[3][4]) {
     float inv_s[3];
     e3 = 0;
     for (int a = 0; a < 3; a++) {
@@ -544,20 +544,18 @@ __device__ __forceinline__ void quantize_node(const Ref& nb, const uint32_t* slo
         ex = max(-100, min(100, ex));
         e3 |= (uint32_t)(ex + 127) << (8 * a);
         inv_s[a] = __uint_as_float((uint32_t)(127 - ex) << 23);
-        qlo[a][0] = qlo[a][1] = qhi[a][0] = qhi[a][1] = 0;
+        q[a][0] = q[a][1] = q[a][2] = q[a][3] = 0;
     }
     for (int sl = 0; sl < 8; sl++) {
         uint32_t c = slots[sl];
         if (c == 0xffffffffu) continue;
         Ref cb = load_ref(c, bvh2, order, tribox);
-        int wsel = sl >> 2, sh = (sl & 3) * 8;
         for (int a = 0; a < 3; a++) {
             float lo = floorf(__fmul_rn(__fsub_rd(cb.lo[a], nb.lo[a]), inv_s[a]));
             float hi = ceilf(__fmul_rn(__fsub_ru(cb.hi[a], nb.lo[a]), inv_s[a]));
             lo = fminf(fmaxf(lo, 0.f), 255.f);
             hi = fminf(fmaxf(hi, 0.f), 255.f);
-            qlo[a][wsel] |= (uint32_t)lo << sh;
-            qhi[a][wsel] |= (uint32_t)hi << sh;
+            q[a][sl >> 1] |= ((uint32_t)lo | ((uint32_t)hi << 8)) << ((sl & 1) * 16);
         }
     }
 }
@@ -579,8 +577,8 @@ __global__ void k_collapse_emit(uint32_t m, uint32_t level_start, uint32_t tri_s
     // kept for refits: the node's BVH2 subtree and its children in slot order
     node_ref[level_start + k] = lvl[k];
     for (int sl = 0; sl < 8; sl++) node_plan[(size_t)(level_start + k) * 8 + sl] = slots[sl];
-    uint32_t e3, qlo[3][2], qhi[3][2];
-    quantize_node(nb, slots, bvh2, order, tribox, e3, qlo, qhi);
+    uint32_t e3, q[3][4];
+    quantize_node(nb, slots, bvh2, order, tribox, e3, q);
     uint32_t imask = 0, meta[2] = {0, 0};
     uint32_t toff = 0, rank = 0;
     for (int sl = 0; sl < 8; sl++) {
@@ -611,9 +609,7 @@ __global__ void k_collapse_emit(uint32_t m, uint32_t level_start, uint32_t tri_s
     nd.q[0] = make_uint4(__float_as_uint(nb.lo[0]), __float_as_uint(nb.lo[1]), __float_as_uint(nb.lo[2]),
                          e3 | (imask << 24));
     nd.q[1] = make_uint4(child_base, tri_base, meta[0], meta[1]);
-    nd.q[2] = make_uint4(qlo[0][0], qlo[0][1], qlo[1][0], qlo[1][1]);
-    nd.q[3] = make_uint4(qlo[2][0], qlo[2][1], qhi[0][0], qhi[0][1]);
-    nd.q[4] = make_uint4(qhi[1][0], qhi[1][1], qhi[2][0], qhi[2][1]);
+    for (int a = 0; a < 3; a++) nd.q[2 + a] = make_uint4(q[a][0], q[a][1], q[a][2], q[a][3]);
     nodes[node_off + level_start + k] = nd;
 }
 
@@ -627,15 +623,13 @@ __global__ void k_requantize(uint32_t n_nodes, const uint32_t* __restrict__ node
     uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n_nodes) return;
     Ref nb = load_ref(node_ref[k], bvh2, order, tribox);
-    uint32_t e3, qlo[3][2], qhi[3][2];
-    quantize_node(nb, node_plan + (size_t)k * 8, bvh2, order, tribox, e3, qlo, qhi);
+    uint32_t e3, q[3][4];
+    quantize_node(nb, node_plan + (size_t)k * 8, bvh2, order, tribox, e3, q);
     Node8& nd = nodes[k];
     const uint32_t imask = nd.q[0].w >> 24;
     nd.q[0] = make_uint4(__float_as_uint(nb.lo[0]), __float_as_uint(nb.lo[1]), __float_as_uint(nb.lo[2]),
                          e3 | (imask << 24));
-    nd.q[2] = make_uint4(qlo[0][0], qlo[0][1], qlo[1][0], qlo[1][1]);
-    nd.q[3] = make_uint4(qlo[2][0], qlo[2][1], qhi[0][0], qhi[0][1]);
-    nd.q[4] = make_uint4(qhi[1][0], qhi[1][1], qhi[2][0], qhi[2][1]);
+    for (int a = 0; a < 3; a++) nd.q[2 + a] = make_uint4(q[a][0], q[a][1], q[a][2], q[a][3]);
 }
 
 // packed triangles take their (new) world vertices by the id they carry

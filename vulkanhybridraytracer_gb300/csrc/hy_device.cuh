@@ -249,15 +249,17 @@ __device__ __forceinline__ void accum_store(uint32_t fmt, void* buf, size_t i, f
 // node words (uint4 q[5]):
 //  q0 = p.x, p.y, p.z, e.x | e.y<<8 | e.z<<16 | imask<<24
 //  q1 = child_base, tri_base, meta[0..3], meta[4..7]
-//  q2 = qlo_x[0..3], qlo_x[4..7], qlo_y[0..3], qlo_y[4..7]
-//  q3 = qlo_z[0..3], qlo_z[4..7], qhi_x[0..3], qhi_x[4..7]
-//  q4 = qhi_y[0..3], qhi_y[4..7], qhi_z[0..3], qhi_z[4..7]
+//  q2, q3, q4 = the x, y, z planes: word j holds the bytes lo, hi of slot 2j and lo, hi
+//               of slot 2j + 1
+// (hy_bvh_download gives each axis's lo bytes of slots 0..7, then its hi bytes, as
+// the words qlo_x, qlo_y, qlo_z, qhi_x, qhi_y, qhi_z of two words each)
 // meta[s]: 0 = empty slot, 0x80 = internal child, else (count << 5) | triangle offset
 // triangle (float4 t[3]) = (v0, id bits), (v1, 0), (v2, 0)
 struct Node8 { uint4 q[5]; };
 constexpr int kLeafMax = 3;
 constexpr int kStackMax = 64;
 constexpr uint32_t kMaxIters = 1u << 22;
+constexpr float kBoxSlack = 1.0000003f;  // box test: tnear <= tfar * kBoxSlack (1 + 3 * 2^-23)
 
 struct SceneDev {
     const Node8* nodes;
@@ -361,11 +363,6 @@ __device__ __forceinline__ bool tri_test(const RayPre& r, float4 v0, float4 v1, 
     return true;
 }
 
-__device__ __forceinline__ uint32_t byte_at(uint32_t lo4, uint32_t hi4, int slot) {
-    uint32_t w = slot < 4 ? lo4 : hi4;
-    return (w >> ((slot & 3) * 8)) & 0xffu;
-}
-
 // three-input max / min (one instruction on sm_100+); NaN inputs are ignored as by fmaxf / fminf
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
     float d;
@@ -384,18 +381,8 @@ __device__ __forceinline__ unsigned long long f2_pack(float a, float b) {
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
     return r;
 }
-__device__ __forceinline__ unsigned long long f2_pack_bits(uint32_t a, uint32_t b) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b));
-    return r;
-}
 __device__ __forceinline__ void f2_unpack(unsigned long long v, float& a, float& b) {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ unsigned long long f2_add(unsigned long long a, unsigned long long b) {
-    unsigned long long d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
 }
 __device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsigned long long b,
                                                      unsigned long long c) {
@@ -408,12 +395,6 @@ __device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsig
 __device__ __forceinline__ void h2_to_f2(uint32_t h, float& lo, float& hi) {
     asm("{ .reg .b16 l, u; mov.b32 {l, u}, %2; cvt.f32.f16 %0, l; cvt.f32.f16 %1, u; }"
         : "=f"(lo), "=f"(hi) : "r"(h));
-}
-
-// bit k set when byte k of hi4:lo4 is nonzero
-__device__ __forceinline__ uint32_t nonzero_bytes(uint32_t lo4, uint32_t hi4) {
-    const uint32_t a = __vcmpne4(lo4, 0u) & 0x80808080u, b = __vcmpne4(hi4, 0u) & 0x80808080u;
-    return ((a * 0x00204081u) >> 28) | (((b * 0x00204081u) >> 28) << 4);
 }
 
 // bit s of an 8-bit slot mask moved to bit s ^ ord (the slots' traversal ranks)
@@ -658,60 +639,55 @@ __device__ __forceinline__ bool trav_node(const SceneDev& S, const RW& rw, float
         org[a] = __fmul_rn(__fsub_rn(p[a], oo[a]), r.invd[a]);
     }
     const uint32_t imask = q0.w >> 24;
-    // near/far planes per axis: a ray going in -a enters through the max plane,
-    // so the quantised lo/hi byte planes swap once per node, not per child
-    uint32_t qn[3][2], qf[3][2];
-    {
-        const uint32_t qlo[3][2] = {{q2.x, q2.y}, {q2.z, q2.w}, {q3.x, q3.y}};
-        const uint32_t qhi[3][2] = {{q3.z, q3.w}, {q4.x, q4.y}, {q4.z, q4.w}};
-#pragma unroll
-        for (int a = 0; a < 3; a++) {
-            const bool neg = r.invd[a] < 0.f;
-#pragma unroll
-            for (int w = 0; w < 2; w++) {
-                qn[a][w] = neg ? qhi[a][w] : qlo[a][w];
-                qf[a][w] = neg ? qlo[a][w] : qhi[a][w];
-            }
-        }
-    }
-    uint32_t hitbits = 0;
-    // Plane bytes as subnormal halves: one PRMT makes 0x00qq:0x00qq, the
-    // halves q * 2^-24 of two slots, whose conversion to float is exact; with
-    // adj scaled by 2^24 (exact) one fma gives q * adj + org rounded once, the
-    // same value as fma(q, adj, org).  Per axis, the (near, far) pair of a
-    // slot is one f32x2 fma.
+    // Plane bytes as subnormal halves: one PRMT makes 0x00qq:0x00qq, the near
+    // and far plane of a slot as the halves q * 2^-24, whose conversion to float
+    // is exact; with adj scaled by 2^24 (exact) one fma gives q * adj + org
+    // rounded once, the same value as fma(q, adj, org).  A ray going in -a enters
+    // through the hi plane: the PRMT's selector (bytes lo, hi of a slot, in the
+    // ray's order) does that for free, and the pair is one f32x2 fma.
+    uint32_t sel[3];
     unsigned long long adj2[3], org2[3];
 #pragma unroll
     for (int a = 0; a < 3; a++) {
+        sel[a] = r.invd[a] < 0.f ? 0x4041u : 0x4140u;
         const float a24 = __fmul_rn(adj[a], 16777216.0f);
         adj2[a] = f2_pack(a24, a24);
         org2[a] = f2_pack(org[a], org[a]);
     }
+    const uint32_t q[3][4] = {{q2.x, q2.y, q2.z, q2.w}, {q3.x, q3.y, q3.z, q3.w}, {q4.x, q4.y, q4.z, q4.w}};
+    // A box is hit when max(tn, tmin) <= rn(min(tf, tmax) * c).  rn(. * c) is
+    // monotone, so that is tn <= rn(tf c), tn <= rn(tmax c), tmin <= rn(tf c) (a
+    // ray has tmin <= tmax): three differences whose signs are exact, gathered by one
+    // three-input OR and one funnel shift per slot.  The differences run on the FMA
+    // pipe; min / max / compare would run on the ALU pipe, which limits the walk.
+    // (NaN planes, 0 * inf, are skipped by max / min, and a difference with NaN
+    // has a clear sign: such a box counts as hit, as with the comparisons.)
+    const float tmaxc = __fmul_rn(t.tmax, kBoxSlack);
+    uint32_t miss = 0;
 #pragma unroll
-    for (int j = 0; j < 4; j++) {  // the slot pair 2j, 2j + 1: bytes (2j) & 3 and the next of word j / 2
-        const uint32_t kSel = (j & 1) ? 0x4342u : 0x4140u;
+    for (int j = 3; j >= 0; j--) {  // slots 2j + 1, 2j: the funnel shift takes the highest slot first
         float tn[2][3], tf[2][3];
 #pragma unroll
         for (int a = 0; a < 3; a++) {
-            float n0, n1, f0, f1;
-            h2_to_f2(__byte_perm(qn[a][j >> 1], 0u, kSel), n0, n1);
-            h2_to_f2(__byte_perm(qf[a][j >> 1], 0u, kSel), f0, f1);
+            float n0, f0, n1, f1;
+            h2_to_f2(__byte_perm(q[a][j], 0u, sel[a]), n0, f0);
+            h2_to_f2(__byte_perm(q[a][j], 0u, sel[a] + 0x0202u), n1, f1);
             f2_unpack(f2_fma(f2_pack(n0, f0), adj2[a], org2[a]), tn[0][a], tf[0][a]);
             f2_unpack(f2_fma(f2_pack(n1, f1), adj2[a], org2[a]), tn[1][a], tf[1][a]);
         }
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            // max(max(tn0, tn1), max(tn2, tmin)) and its min twin, as two instructions each
-            const float tnear = fmaxf(fmax3(tn[h][0], tn[h][1], tn[h][2]), tmin);
-            const float tfar = fminf(fmin3(tf[h][0], tf[h][1], tf[h][2]), t.tmax);
-            if (tnear <= __fmul_rn(tfar, 1.0000003f)) hitbits |= 1u << (2 * j + h);
+        for (int h = 1; h >= 0; h--) {
+            const float tnear = fmax3(tn[h][0], tn[h][1], tn[h][2]);
+            const float m = __fmul_rn(fmin3(tf[h][0], tf[h][1], tf[h][2]), kBoxSlack);
+            const uint32_t out = __float_as_uint(__fsub_rn(m, tnear)) | __float_as_uint(__fsub_rn(tmaxc, tnear)) |
+                                 __float_as_uint(__fsub_rn(m, tmin));
+            miss = __funnelshift_l(out, miss, 1);
         }
     }
-    // empty slots (meta byte 0) never count; internal children go to the stack
-    // in rank order, leaf slots give their triangles
-    hitbits &= nonzero_bytes(q1.z, q1.w);
-    const uint32_t hit_int = slots_to_ranks(hitbits & imask, ord);
-    uint32_t hit_leaf = hitbits & ~imask, hit_tri = 0;
+    // internal children go to the stack in rank order, leaf slots give their
+    // triangles (an empty slot, whose box is the node's lo corner, has none)
+    const uint32_t hit_int = slots_to_ranks(~miss & imask, ord);
+    uint32_t hit_leaf = ~(miss | imask) & 0xffu, hit_tri = 0;
     while (hit_leaf) {
         const uint32_t slot = __ffs(hit_leaf) - 1;
         hit_leaf &= hit_leaf - 1u;

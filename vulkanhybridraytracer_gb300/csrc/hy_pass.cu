@@ -504,8 +504,10 @@ __global__ void __launch_bounds__(128) k_trace(const SceneDev S, const HyRay* __
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i - threadIdx.x < n; i += gridDim.x * blockDim.x) {
         if (i < n) {
             HyRay r = rays[i];
+            // an empty interval enters no box (the walk's box test takes tmin <= tmax for granted)
+            const float tmax = r.tmin > __fmul_rn(r.tmax, kBoxSlack) ? -INFINITY : r.tmax;
             Hit h = trace<ANY, COUNT>(S, mk(r.org[0], r.org[1], r.org[2]), mk(r.dir[0], r.dir[1], r.dir[2]), r.tmin,
-                                      r.tmax, ls, status);
+                                      tmax, ls, status);
             ls.shadow++;
             HyHit o;
             o.t = h.id == HY_NO_HIT ? 0.f : h.t;
