@@ -307,15 +307,17 @@ PassParams make_params(HyCtx* c, const HyGBuffer* gb, const HyCamera* cam, const
 }
 
 // ---- per-kernel timing ----
-// the first seven are the MODE_* values of hy_pass.h
-enum { PK_ACCUM = MODE_SHADOW_ACCUM_S + 1, PK_GRAD, PK_PATHTRACE, PK_COUNT };
+// the first are the MODE_* values of hy_pass.h
+enum { PK_ACCUM = MODE_SHADOW_ACCUM_S1 + 1, PK_GRAD, PK_PATHTRACE, PK_COUNT };
 const char* const kProfNames[PK_COUNT] = {"k_shadow",       "k_pixels<shade>",       "k_shadow<accum>",
                                           "k_shadow_group", "k_shadow_group<accum>", "k_shadow_pool",
                                           "k_shadow_pool<accum>", "k_shadow_stream", "k_shadow_stream<accum>",
+                                          "k_shadow_stream<one>", "k_shadow_stream<accum, one>",
                                           "k_accumulate", "k_shade_grad", "k_pathtrace"};
 static_assert(MODE_SHADOW == 0 && MODE_SHADE == 1 && MODE_SHADOW_ACCUM == 2 && MODE_SHADOW_G == 3 &&
                   MODE_SHADOW_ACCUM_G == 4 && MODE_SHADOW_P == 5 && MODE_SHADOW_ACCUM_P == 6 &&
-                  MODE_SHADOW_S == 7 && MODE_SHADOW_ACCUM_S == 8,
+                  MODE_SHADOW_S == 7 && MODE_SHADOW_ACCUM_S == 8 && MODE_SHADOW_S1 == 9 &&
+                  MODE_SHADOW_ACCUM_S1 == 10,
               "profile names follow the pass modes");
 
 cudaEvent_t prof_event(HyCtx* c) {
@@ -358,7 +360,9 @@ int run_pixels(HyCtx* c, int mode, const PassParams& P0, const HyPassConfig* cfg
     if ((mode == MODE_SHADOW || mode == MODE_SHADOW_ACCUM) && !(cfg->flags & HY_FLAG_PIXEL_PARALLEL)) {
         if (sampled && (cfg->flags & HY_FLAG_RAY_POOL)) {
             mode = mode == MODE_SHADOW ? MODE_SHADOW_P : MODE_SHADOW_ACCUM_P;
-        } else if (!sampled || !(cfg->flags & HY_FLAG_LANE_GROUPS)) {
+        } else if (!sampled) {
+            mode = mode == MODE_SHADOW ? MODE_SHADOW_S1 : MODE_SHADOW_ACCUM_S1;
+        } else if (!(cfg->flags & HY_FLAG_LANE_GROUPS)) {
             mode = mode == MODE_SHADOW ? MODE_SHADOW_S : MODE_SHADOW_ACCUM_S;
         } else {
             mode = mode == MODE_SHADOW ? MODE_SHADOW_G : MODE_SHADOW_ACCUM_G;
@@ -374,7 +378,7 @@ int run_pixels(HyCtx* c, int mode, const PassParams& P0, const HyPassConfig* cfg
     // measured fastest on the 1080p workload: 6 resident blocks (80 registers)
     // for the lane-group kernel (1.4 % ahead of 8), 8 (64 registers) otherwise
     const bool grouped = mode == MODE_SHADOW_G || mode == MODE_SHADOW_ACCUM_G;
-    const bool streams = mode == MODE_SHADOW_S || mode == MODE_SHADOW_ACCUM_S;
+    const bool streams = mode >= MODE_SHADOW_S;
     int minb = cfg->min_blocks ? (int)cfg->min_blocks : (grouped ? 6 : 8);
     if (streams && !cfg->visits_per_round) P.inner = kStreamSteps;
     if (cfg->stack_depth && cfg->stack_depth != 8) return HY_ERR_UNSUPPORTED;

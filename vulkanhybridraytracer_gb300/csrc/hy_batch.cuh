@@ -67,18 +67,22 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_shadow_batch_stream(const Batch
         const bool accum = !(P.flags & HY_FLAG_NO_ACCUM) && P.accum_frame > 0;
         const bool reference = P.rng_mode == HY_RNG_REFERENCE;
         const uint32_t tile = unit - P.tile_begin;
+        const bool one = reference || P.spp == 1;  // one ray per pixel and light
+        WalkAreaT<ANY_TWO>& own = sm.scratch[warp].walk;
         if constexpr (ANY_TWO) {  // compiled without a shared stack
             if (S.two_level) {
                 WorldRaySlot w{s_world + threadIdx.x, &sm.scratch[warp].walk.ray[lane]};
-                stream_tile<COUNT, true, 2>(S, P, tile, reference, accum, sm, stk, t, w, s, ls, nn, nt);
+                if (one) stream_tile_one<COUNT, true, 2>(S, P, tile, reference, accum, own, stk, t, w, s, ls, nn, nt);
+                else stream_tile<COUNT, true, 2>(S, P, tile, reference, accum, sm, stk, t, w, s, ls, nn, nt);
                 continue;
             }
         }
-        if constexpr (SHORT > 0)
-            stream_tile<COUNT, false, 2>(S, P, tile, reference, accum, sm,
-                                         SplitStackT<SHORT, BLOCK>{s_stack + threadIdx.x, stk}, t, r, s, ls, nn, nt);
-        else
-            stream_tile<COUNT, false, 2>(S, P, tile, reference, accum, sm, stk, t, r, s, ls, nn, nt);
+        auto run = [&](auto stack) {
+            if (one) stream_tile_one<COUNT, false, 2>(S, P, tile, reference, accum, own, stack, t, r, s, ls, nn, nt);
+            else stream_tile<COUNT, false, 2>(S, P, tile, reference, accum, sm, stack, t, r, s, ls, nn, nt);
+        };
+        if constexpr (SHORT > 0) run(SplitStackT<SHORT, BLOCK>{s_stack + threadIdx.x, stk});
+        else run((uint2*)stk);
     }
     if (COUNT) { ls.nodes += nn; ls.tris += nt; }
     flush_stats(ls, B.stats);

@@ -1006,10 +1006,12 @@ static void* shade_kernel(bool count, int minb, bool two) {
 }
 
 static void* pixel_kernel(int mode, bool count, int minb, bool two, bool short_stack = false, int shade_minb = 0) {
-    if (mode == MODE_SHADOW_S || mode == MODE_SHADOW_ACCUM_S) {
-        const bool accum = mode == MODE_SHADOW_ACCUM_S;
-        if (two) return stream_kernel_two(accum, count);
-        return accum ? stream_kernel_accum(count, minb, short_stack) : stream_kernel_raw(count, minb, short_stack);
+    if (mode >= MODE_SHADOW_S) {
+        const bool accum = mode == MODE_SHADOW_ACCUM_S || mode == MODE_SHADOW_ACCUM_S1;
+        const bool one = mode == MODE_SHADOW_S1 || mode == MODE_SHADOW_ACCUM_S1;
+        if (two) return stream_kernel_two(accum, count, one);
+        return accum ? stream_kernel_accum(count, minb, short_stack, one)
+                     : stream_kernel_raw(count, minb, short_stack, one);
     }
     if (two) {
         switch (mode) {

@@ -8,10 +8,12 @@
 namespace hy {
 
 // *_G: the sample-parallel shadow kernel (DECORRELATED rays, spp >= 2) with lane
-// groups per pixel-light; *_P: the same rays from a per-warp ray pool
+// groups per pixel-light; *_P: the same rays from a per-warp ray pool; *_S: tile
+// streams; *_S1: tile streams with one ray per pixel and light
 enum {
     MODE_SHADOW = 0, MODE_SHADE = 1, MODE_SHADOW_ACCUM = 2, MODE_SHADOW_G = 3, MODE_SHADOW_ACCUM_G = 4,
-    MODE_SHADOW_P = 5, MODE_SHADOW_ACCUM_P = 6, MODE_SHADOW_S = 7, MODE_SHADOW_ACCUM_S = 8
+    MODE_SHADOW_P = 5, MODE_SHADOW_ACCUM_P = 6, MODE_SHADOW_S = 7, MODE_SHADOW_ACCUM_S = 8,
+    MODE_SHADOW_S1 = 9, MODE_SHADOW_ACCUM_S1 = 10
 };
 
 struct PassParams {
@@ -116,9 +118,9 @@ cudaError_t launch_batch(bool shade, bool count, int minb, bool stream, bool two
 cudaError_t batch_occupancy(bool shade, bool count, int minb, bool stream, bool two, int block, int shortd,
                             int* blocks_per_sm);
 // tile-stream shadow kernels (hy_stream_raw.cu, hy_stream_accum.cu, hy_stream_two.cu)
-void* stream_kernel_raw(bool count, int minb, bool short_stack);
-void* stream_kernel_accum(bool count, int minb, bool short_stack);
-void* stream_kernel_two(bool accum, bool count);
+void* stream_kernel_raw(bool count, int minb, bool short_stack, bool one);
+void* stream_kernel_accum(bool count, int minb, bool short_stack, bool one);
+void* stream_kernel_two(bool accum, bool count, bool one);
 void* batch_stream_kernel_64(bool count, int minb, int shortd, bool two);
 void* batch_stream_kernel_128(bool count, int minb, int shortd, bool two);
 void* batch_stream_kernel_256(bool count, int minb, int shortd, bool two);

@@ -33,6 +33,18 @@ namespace hy {
 // kernel (instance ids per pair, 3 KB of world rays) takes the 164 KB step.
 constexpr uint32_t kSortItems = 512, kSortBuckets = 64;
 constexpr uint32_t kPairs = 64;  // (ray, triangle) pairs a warp collects between two test phases
+
+// A warp's walk: each lane's ray (direction, tmax) and the (ray, triangle) pairs
+// waiting for their test.
+template <bool TWO>
+struct WalkAreaT {
+    float4 ray[32];
+    uint32_t rec[kPairs];             // triangle record
+    uint32_t inst[TWO ? kPairs : 1];  // two-level: its instance
+    uint8_t owner[kPairs];            // the lane whose ray it is
+    uint32_t npairs;                  // pairs collected (may count past kPairs: those wait on their lanes)
+};
+
 template <int NW, bool TWO = false, uint32_t SORT = kSortItems>  // warps per block, items sorted together
 struct StreamSlotsT {
     static constexpr uint32_t kSort = SORT;
@@ -41,20 +53,13 @@ struct StreamSlotsT {
     float4 T[NW * 32];
     float4 B[NW * 32];
     uint16_t order[NW][SORT];  // per warp: the traced items of the light ordered by their disk sample
-    uint32_t npairs[NW];       // per warp: pairs collected (may count past kPairs: those wait on their lanes)
     union Scratch {
         // the sort: the sample's cell per item, the cell counts / cursors
         struct {
             uint8_t key[SORT];
             uint32_t bucket[kSortBuckets];
         } sort;
-        // the walk: each lane's ray (direction, tmax) and the pairs waiting for their test
-        struct {
-            float4 ray[32];
-            uint32_t rec[kPairs];
-            uint32_t inst[TWO ? kPairs : 1];
-            uint8_t owner[kPairs];
-        } walk;
+        WalkAreaT<TWO> walk;
     };
     alignas(16) Scratch scratch[NW];
 };
@@ -87,11 +92,10 @@ __device__ __forceinline__ void stream_publish(Slots& sm, bool traced, f3 positi
 
 // The triangles of the leaf slots a lane's last node visit hit, put into the
 // warp's pair list; what does not fit stays in t.pend_bits.
-template <bool TWO, class Slots>
-__device__ __forceinline__ void pairs_push(Slots& sm, Trav& t) {
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    auto& w = sm.scratch[warp].walk;
-    uint32_t at = atomicAdd(&sm.npairs[warp], (uint32_t)__popc(t.pend_bits));
+template <bool TWO, class Area>
+__device__ __forceinline__ void pairs_push(Area& w, Trav& t) {
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t at = atomicAdd(&w.npairs, (uint32_t)__popc(t.pend_bits));
     while (t.pend_bits && at < kPairs) {
         const uint32_t b = __ffs(t.pend_bits) - 1;
         t.pend_bits &= t.pend_bits - 1u;
@@ -106,11 +110,10 @@ __device__ __forceinline__ void pairs_push(Slots& sm, Trav& t) {
 // owner (origin by shuffle, direction and tmax from the owner's slot; two-level:
 // moved into the pair's instance) and sets it up for the test as the owner would
 // have.  Returns the mask of owners with a hit.  All lanes call it, np uniform.
-template <bool TWO, class Slots, class RW>
-__device__ __forceinline__ uint32_t pairs_test(const SceneDev& S, Slots& sm, uint32_t np, const RW& r, float tmin,
+template <bool TWO, class Area, class RW>
+__device__ __forceinline__ uint32_t pairs_test(const SceneDev& S, const Area& w, uint32_t np, const RW& r, float tmin,
                                                uint32_t* status) {
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const auto& w = sm.scratch[warp].walk;
+    const uint32_t lane = threadIdx.x & 31;
     uint32_t hits = 0;
     for (uint32_t b = 0; b < np; b += 32) {
         const uint32_t i = b + lane;
@@ -144,18 +147,14 @@ __device__ __forceinline__ uint32_t pairs_test(const SceneDev& S, Slots& sm, uin
     return __reduce_or_sync(0xffffffffu, hits);
 }
 
-// The warp's items of one light (every lane calls it, after all lanes have
-// published): sample k of a pixel starts from its first state advanced 2k LCG
-// steps (sampleDisk's two draws per sample), its ray from position +
-// offset * dir to distance + 1.  On return unocc_count holds each pixel's
-// unoccluded samples.
+// One round of a warp's walks: up to P.inner node visits per lane, then the
+// triangles those visits reached, tested together.  All lanes call it; a lane with a
+// ray (live) gets whether the ray is done and whether it is occluded.
 //
-// A round is: idle lanes take the light's next items; up to P.inner node visits
-// per lane; the triangles those visits reached, tested together.  A lane does
-// not test its triangles where it finds them: it puts (ray, triangle) pairs into
-// the warp's list and walks on, and at the end of the round the warp's lanes take
-// one pair each.  On the 1080p frame a node visit of the warp reaches 2.5
-// triangles, on 2.5 lanes: tested at once they took as many warp instructions
+// A lane does not test its triangles where it finds them: it puts (ray, triangle)
+// pairs into the warp's list and walks on, and at the end of the round the warp's
+// lanes take one pair each.  On the 1080p frame a node visit of the warp reaches
+// 2.5 triangles, on 2.5 lanes: tested at once they took as many warp instructions
 // as a third of the whole kernel; collected over a round they fill the lanes
 // (4.85 -> 4.27 G warp instructions on the 960x540 frame, 15.5 -> 20.2 lanes each;
 // 1080p shadow kernel 20.1 -> 17.9 ms, 1277x719 two-level 16.3 -> 13.0 ms).
@@ -167,6 +166,56 @@ __device__ __forceinline__ uint32_t pairs_test(const SceneDev& S, Slots& sm, uin
 // (node visits, stack) is reported only if none of the ray's waiting pairs hit.
 // COUNT: the plain walk, each visit's triangles tested at once, so the counts are
 // those of each ray's walk up to its first hit.
+struct RoundResult { bool over, occluded; };
+template <bool COUNT, bool TWO, class Area, class Stack, class RW>
+__device__ __forceinline__ RoundResult stream_round(const SceneDev& S, const PassParams& P, Area& w, bool live,
+                                                    Stack stk, Trav& t, RW& r, uint32_t& nn, uint32_t& nt) {
+    const uint32_t lane = threadIdx.x & 31;
+    RoundResult res{false, false};
+    uint32_t limits = 0;
+    if (live) {
+        for (uint32_t it = 0, ni = max(P.inner, 1u); it < ni; it++) {
+            if constexpr (COUNT) {
+                if (trav_step<true, true, TWO>(S, r, 0.001f, t, stk, nn, nt, P.status)) {
+                    res.over = true;
+                    res.occluded = t.h.id != HY_NO_HIT;
+                    break;
+                }
+            } else {
+                if (trav_node<true, false, TWO>(S, r, 0.001f, t, stk, nn, DeferredStatus{limits})) {
+                    res.over = true;
+                    break;
+                }
+                if (t.pend_bits) {
+                    pairs_push<TWO>(w, t);
+                    if (t.pend_bits) break;  // the list is full: the rest after the test below
+                }
+            }
+        }
+    }
+    if constexpr (!COUNT) {
+        for (;;) {
+            __syncwarp();
+            const uint32_t np = min(w.npairs, kPairs);
+            if (np == 0) break;
+            const uint32_t hits = pairs_test<TWO>(S, w, np, r, 0.001f, P.status);
+            if (lane == 0) w.npairs = 0;
+            if ((hits >> lane) & 1u) { res.occluded = true; t.pend_bits = 0; }
+            __syncwarp();
+            if (__ballot_sync(0xffffffffu, live && t.pend_bits != 0) == 0) break;
+            if (live && t.pend_bits) pairs_push<TWO>(w, t);
+        }
+    }
+    if (limits && !res.occluded) atomicOr(P.status, limits);
+    res.over = res.over || res.occluded;
+    return res;
+}
+
+// The warp's items of one light (every lane calls it, after all lanes have
+// published): sample k of a pixel starts from its first state advanced 2k LCG
+// steps (sampleDisk's two draws per sample), its ray from position +
+// offset * dir to distance + 1.  On return unocc_count holds each pixel's
+// unoccluded samples.
 template <bool COUNT, bool TWO, class Stack, class Slots, class RW>
 __device__ __forceinline__ void stream_light(const SceneDev& S, const PassParams& P, Slots& sm, uint32_t nrays,
                                              float radius, float offset, Stack stk, Trav& t, RW& r,
@@ -229,7 +278,8 @@ __device__ __forceinline__ void stream_light(const SceneDev& S, const PassParams
                 if (key != 0xffu) sm.order[warp][atomicAdd(&bk[key], 1u)] = (uint16_t)j;
             }
         }
-        if (lane == 0) sm.npairs[warp] = 0;
+        __syncwarp();  // the sort's scratch becomes the walk's
+        if (lane == 0) sm.scratch[warp].walk.npairs = 0;
         __syncwarp();
         bool live = false;
         uint32_t cur = 0, head = 0;  // head: the first unclaimed item (the same on every lane)
@@ -260,49 +310,10 @@ __device__ __forceinline__ void stream_light(const SceneDev& S, const PassParams
             } else if (idle == 0xffffffffu) {
                 break;
             }
-            // ---- up to P.inner node visits ----
-            bool over = false, occluded = false;
-            uint32_t limits = 0;
-            if (live) {
-                for (uint32_t it = 0, ni = max(P.inner, 1u); it < ni; it++) {
-                    if constexpr (COUNT) {
-                        if (trav_step<true, true, TWO>(S, r, 0.001f, t, stk, nn, nt, P.status)) {
-                            over = true;
-                            occluded = t.h.id != HY_NO_HIT;
-                            break;
-                        }
-                    } else {
-                        if (trav_node<true, false, TWO>(S, r, 0.001f, t, stk, nn, DeferredStatus{limits})) {
-                            over = true;
-                            break;
-                        }
-                        if (t.pend_bits) {
-                            pairs_push<TWO>(sm, t);
-                            if (t.pend_bits) break;  // the list is full: the rest after the test below
-                        }
-                    }
-                }
-            }
-            // ---- the round's triangles ----
-            if constexpr (!COUNT) {
-                for (;;) {
-                    __syncwarp();
-                    const uint32_t np = min(sm.npairs[warp], kPairs);
-                    if (np == 0) break;
-                    const uint32_t hits = pairs_test<TWO>(S, sm, np, r, 0.001f, P.status);
-                    if (lane == 0) sm.npairs[warp] = 0;
-                    if ((hits >> lane) & 1u) { occluded = true; t.pend_bits = 0; }
-                    __syncwarp();
-                    if (__ballot_sync(0xffffffffu, live && t.pend_bits != 0) == 0) break;
-                    if (live && t.pend_bits) pairs_push<TWO>(sm, t);
-                }
-            }
-            if (live && (over || occluded)) {
+            const RoundResult res = stream_round<COUNT, TWO>(S, P, sm.scratch[warp].walk, live, stk, t, r, nn, nt);
+            if (live && res.over) {
                 live = false;
-                if (!occluded) {
-                    if (limits) atomicOr(P.status, limits);
-                    atomicAdd(unocc_count(sm, wb + cur), 1u);
-                }
+                if (!res.occluded) atomicAdd(unocc_count(sm, wb + cur), 1u);
             }
         }
         __syncwarp();
@@ -336,6 +347,21 @@ __device__ __forceinline__ void shadow_finalize(const PassParams& P, const Shado
     }
 }
 
+// a lane's pixel: its G-buffer texel and the RNG state of its first sample
+__device__ __forceinline__ void stream_pixel(const SceneDev& S, const PassParams& P, uint32_t x, uint32_t y,
+                                             ShadowLane& s) {
+    s.pix = y * P.W + x;
+    const float4 g0 = fetch_texel(P.plane[0], P.fmt[0], s.pix);
+    const float4 g1 = fetch_texel(P.plane[1], P.fmt[1], s.pix);
+    s.position = mk(g0.x, g0.y, g0.z);
+    s.N = normalize_rn(mk(__fsub_rn(__fmul_rn(g1.x, 2.0f), 1.0f), __fsub_rn(__fmul_rn(g1.y, 2.0f), 1.0f),
+                          __fsub_rn(__fmul_rn(g1.z, 2.0f), 1.0f)));
+    const int mi = mat_index(g0.w, S.num_mats);
+    s.smode = mi >= 0 ? (int)S.mats[mi].smr[0] : 0;
+    s.seed = tea(s.pix, P.frame_u);
+    s.in_blur = x < P.blur_w && y < P.blur_h;
+}
+
 // ---------------------------------------------------------------------------------
 // One 8x4 tile of a view, light by light.  ACC: 0 raw shadow images, 1 the
 // running mean into the history, 2 either (accum) at run time.  reference:
@@ -355,16 +381,8 @@ __device__ __forceinline__ void stream_tile(const SceneDev& S, const PassParams&
     };
     uint32_t seed0 = 0, rays_before = 0;
     if (present) {
-        s.pix = y * P.W + x;
-        const float4 g0 = fetch_texel(P.plane[0], P.fmt[0], s.pix);
-        const float4 g1 = fetch_texel(P.plane[1], P.fmt[1], s.pix);
-        s.position = mk(g0.x, g0.y, g0.z);
-        s.N = normalize_rn(mk(__fsub_rn(__fmul_rn(g1.x, 2.0f), 1.0f), __fsub_rn(__fmul_rn(g1.y, 2.0f), 1.0f),
-                              __fsub_rn(__fmul_rn(g1.z, 2.0f), 1.0f)));
-        const int mi = mat_index(g0.w, S.num_mats);
-        s.smode = mi >= 0 ? (int)S.mats[mi].smr[0] : 0;
-        s.in_blur = x < P.blur_w && y < P.blur_h;
-        seed0 = tea(s.pix, P.frame_u);
+        stream_pixel(S, P, x, y, s);
+        seed0 = s.seed;
     }
     for (uint32_t l = 0; l < P.num_lights; l++) {
         // ---- light l for this lane's pixel ----
@@ -393,6 +411,86 @@ __device__ __forceinline__ void stream_tile(const SceneDev& S, const PassParams&
         }
         if (traced) rays_before += spp;
         __syncwarp();  // the slots are rewritten by the next light's set-up
+    }
+}
+
+// The same tile with one ray per pixel and light (REFERENCE RNG, or one sample).
+// A light then gives the warp 32 rays at most, and taking the lights one by one
+// every lane would wait for each light's longest ray (17.8 of 32 lanes walking on
+// the 4K frame with 64 lights).  Here a lane walks its own pixel's rays, light
+// after light, without waiting for the others.  The ray's set-up (light geometry,
+// disk sample) costs two node visits, so it runs on many lanes at a time: when
+// kSetupLanes lanes have nothing to walk, every lane whose slot is free prepares
+// its pixel's next traced light, the walking lanes ahead of time.  Lanes stay
+// within kLightDrift lights of the last one, so that their rays go the same way.
+// Each pixel's lights keep their order, so the RNG states are the sequential loop's.
+constexpr uint32_t kSetupLanes = 16, kLightDrift = 8;
+template <bool COUNT, bool TWO, int ACC, class Area, class Stack, class RW>
+__device__ __forceinline__ void stream_tile_one(const SceneDev& S, const PassParams& P, uint32_t tile, bool reference,
+                                                bool accum, Area& w, Stack stk, Trav& t, RW& r, ShadowLane& s,
+                                                LaneStats& ls, uint32_t& nn, uint32_t& nt) {
+    const uint32_t lane = threadIdx.x & 31;
+    const size_t plane = (size_t)P.W * P.H;
+    const uint32_t x = (tile % P.tiles_x) * 8 + (lane & 7), y = (tile / P.tiles_x) * 4 + (lane >> 3);
+    auto finalize = [&](uint32_t l, float v) {
+        s.light = l;
+        if (ACC == 0 || (ACC == 2 && !accum)) shadow_finalize<false>(P, s, plane, v);
+        else shadow_finalize<true>(P, s, plane, v);
+    };
+    uint32_t next = P.num_lights;  // the pixel's next light to set up
+    if (x < P.W && y < P.H) {
+        stream_pixel(S, P, x, y, s);
+        next = 0;
+    }
+    bool live = false, ready = false;       // walking a ray; a prepared one waits
+    uint32_t light = 0, ready_light = 0;    // their lights
+    f3 ready_dir = mk(0.f, 0.f, 0.f);       // the prepared ray
+    float ready_tmax = 0.f;
+    __syncwarp();
+    if (lane == 0) w.npairs = 0;
+    __syncwarp();
+    for (;;) {
+        const uint32_t starved = __ballot_sync(0xffffffffu, !live && !ready && next < P.num_lights);
+        if (starved && ((uint32_t)__popc(starved) >= kSetupLanes || __ballot_sync(0xffffffffu, live || ready) == 0)) {
+            const uint32_t last = __reduce_min_sync(0xffffffffu, live ? light : (ready ? ready_light : next));
+            while (!ready && next < P.num_lights && next - last <= kLightDrift) {
+                const uint32_t l = next++;
+                const HyLight& lt = S.lights[l];
+                const LightGeo lg = light_geo(lt, s.position, s.N);
+                float v = -1.f;
+                if (s.smode == 4) v = 1.0f;
+                else if (!(lg.NdotL > 0.f)) v = 0.0f;
+                else if (!(lg.dist < lg.maxd)) v = 1.0f;
+                if (v >= 0.f) {
+                    finalize(l, v);
+                    continue;
+                }
+                uint32_t seed = s.seed;
+                ready_dir = sampleDisk(lt.radius, s.position, lg.L, seed);
+                ready_tmax = __fadd_rn(lg.dist, 1.0f);
+                if (!reference) s.seed = seed;  // REFERENCE: sampleDisk takes the pixel's seed by value
+                ready = true;
+                ready_light = l;
+                ls.shadow++;
+            }
+        }
+        if (!live && ready) {
+            w.ray[lane] = make_float4(ready_dir.x, ready_dir.y, ready_dir.z, ready_tmax);
+            // shadowRaygen.rgen:78: origin position + 0.1 dir, tmax distance + 1
+            trav_init(t, world_set(r, add_rn(s.position, scale_rn(ready_dir, 1e-1f)), ready_dir), ready_tmax);
+            light = ready_light;
+            live = true;
+            ready = false;
+        }
+        if (__ballot_sync(0xffffffffu, live) == 0) {
+            if (__ballot_sync(0xffffffffu, next < P.num_lights) == 0) break;
+            continue;
+        }
+        const RoundResult res = stream_round<COUNT, TWO>(S, P, w, live, stk, t, r, nn, nt);
+        if (live && res.over) {
+            live = false;
+            finalize(light, res.occluded ? 0.0f : 1.0f);
+        }
     }
 }
 

@@ -3,7 +3,7 @@
 #include "hy_stream_kernel.cuh"
 
 namespace hy {
-void* stream_kernel_accum(bool count, int minb, bool short_stack) {
-    return stream_kernel_one<true>(count, minb, short_stack);
+void* stream_kernel_accum(bool count, int minb, bool short_stack, bool one) {
+    return stream_kernel_flat<true>(count, minb, short_stack, one);
 }
 }  // namespace hy

@@ -33,9 +33,14 @@ namespace hy {
 // adjacent pixels of one light.  Seeds as in k_shadow_group (LCG jump-ahead),
 // so the rays equal those of k_shadow.
 // ---------------------------------------------------------------------------------
-template <bool COUNT, bool ACCUM, int MINB, bool TWO = false, bool SHORT = false>
+// ONE: one ray per pixel and light (stream_tile_one).
+template <bool TWO>
+struct OneRayBlockT {
+    WalkAreaT<TWO> warp[4];
+};
+template <bool COUNT, bool ACCUM, int MINB, bool TWO = false, bool SHORT = false, bool ONE = false>
 __global__ void __launch_bounds__(128, MINB) k_shadow_stream(const SceneDev S, const PassParams P) {
-    __shared__ StreamSlotsT<4, TWO> sm;
+    __shared__ std::conditional_t<ONE, OneRayBlockT<TWO>, StreamSlotsT<4, TWO>> sm;
     __shared__ uint2 s_stack[SHORT ? kShortStack * 128 : 1];
     __shared__ float s_world[TWO ? 6 * 128 : 1];  // two-level: WorldRaySlot words
     LaneStats ls;
@@ -46,7 +51,8 @@ __global__ void __launch_bounds__(128, MINB) k_shadow_stream(const SceneDev S, c
     std::conditional_t<TWO, WorldRaySlot, RayPre> r{};
     if constexpr (TWO) {
         r.p = s_world + threadIdx.x;
-        r.ray = &sm.scratch[threadIdx.x >> 5].walk.ray[lane];
+        if constexpr (ONE) r.ray = &sm.warp[threadIdx.x >> 5].ray[lane];
+        else r.ray = &sm.scratch[threadIdx.x >> 5].walk.ray[lane];
     }
     uint32_t chunk_cur = 0, chunk_end = 0, nn = 0, nt = 0;
     for (;;) {
@@ -58,21 +64,28 @@ __global__ void __launch_bounds__(128, MINB) k_shadow_stream(const SceneDev S, c
             chunk_cur = t0;
             chunk_end = min(t0 + P.chunk, P.ntiles);
         }
-        if (SHORT)
-            stream_tile<COUNT, TWO, ACCUM ? 1 : 0>(S, P, chunk_cur++, P.rng_mode == HY_RNG_REFERENCE, ACCUM, sm,
+        const bool reference = P.rng_mode == HY_RNG_REFERENCE;
+        if constexpr (ONE)
+            stream_tile_one<COUNT, TWO, ACCUM ? 1 : 0>(S, P, chunk_cur++, reference, ACCUM, sm.warp[threadIdx.x >> 5],
+                                                       stk, t, r, s, ls, nn, nt);
+        else if constexpr (SHORT)
+            stream_tile<COUNT, TWO, ACCUM ? 1 : 0>(S, P, chunk_cur++, reference, ACCUM, sm,
                                                    SplitStack{s_stack + threadIdx.x, stk}, t, r, s, ls, nn, nt);
         else
-            stream_tile<COUNT, TWO, ACCUM ? 1 : 0>(S, P, chunk_cur++, P.rng_mode == HY_RNG_REFERENCE, ACCUM, sm, stk, t,
-                                                   r, s, ls, nn, nt);
+            stream_tile<COUNT, TWO, ACCUM ? 1 : 0>(S, P, chunk_cur++, reference, ACCUM, sm, stk, t, r, s, ls, nn, nt);
     }
     if (COUNT) { ls.nodes += nn; ls.tris += nt; }
     flush_stats(ls, P.stats);
 }
 
 // one-level kernels: the register cap as resident 128-thread blocks per SM
-// (5-8), or 8 with the first stack entries in shared memory
+// (5-8), or 8 with the first stack entries in shared memory; one ray per pixel and
+// light: 8 blocks, the stack in local memory
 template <bool ACCUM>
-static void* stream_kernel_one(bool count, int minb, bool short_stack) {
+static void* stream_kernel_flat(bool count, int minb, bool short_stack, bool one) {
+    if (one)
+        return count ? (void*)k_shadow_stream<true, ACCUM, 8, false, false, true>
+                     : (void*)k_shadow_stream<false, ACCUM, 8, false, false, true>;
     if (short_stack)
         return count ? (void*)k_shadow_stream<true, ACCUM, 8, false, true>
                      : (void*)k_shadow_stream<false, ACCUM, 8, false, true>;

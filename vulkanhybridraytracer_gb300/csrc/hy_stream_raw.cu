@@ -2,5 +2,7 @@
 #include "hy_stream_kernel.cuh"
 
 namespace hy {
-void* stream_kernel_raw(bool count, int minb, bool short_stack) { return stream_kernel_one<false>(count, minb, short_stack); }
+void* stream_kernel_raw(bool count, int minb, bool short_stack, bool one) {
+    return stream_kernel_flat<false>(count, minb, short_stack, one);
+}
 }  // namespace hy

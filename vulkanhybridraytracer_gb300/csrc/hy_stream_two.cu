@@ -4,8 +4,13 @@
 #include "hy_stream_kernel.cuh"
 
 namespace hy {
-void* stream_kernel_two(bool accum, bool count) {
-    if (accum) return count ? (void*)k_shadow_stream<true, true, 8, true> : (void*)k_shadow_stream<false, true, 8, true>;
-    return count ? (void*)k_shadow_stream<true, false, 8, true> : (void*)k_shadow_stream<false, false, 8, true>;
+template <bool ACCUM, bool ONE>
+static void* two_kernel(bool count) {
+    return count ? (void*)k_shadow_stream<true, ACCUM, 8, true, false, ONE>
+                 : (void*)k_shadow_stream<false, ACCUM, 8, true, false, ONE>;
+}
+void* stream_kernel_two(bool accum, bool count, bool one) {
+    if (accum) return one ? two_kernel<true, true>(count) : two_kernel<true, false>(count);
+    return one ? two_kernel<false, true>(count) : two_kernel<false, false>(count);
 }
 }  // namespace hy
