@@ -59,3 +59,30 @@ def test_one_ray_streams_equal_per_pixel_walk(gpu_lib, n_lights, rng_mode, spp, 
         assert torch.equal(hists[0], outs[0][1]) and torch.equal(hists[1], outs[0][1])
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("w,h", [(1, 1), (64, 40), (1100, 700)])
+@pytest.mark.parametrize("n_lights,spp", [(2, 1), (3, 4), (9, 3)])
+def test_light_parts_equal_whole_tiles(gpu_lib, w, h, n_lights, spp):
+    """The last tiles of a launch are handed out in parts of a tile's lights: frames that are
+    all parts and frames that start with whole tiles write the same images as one lane
+    per pixel (the RNG of a part's first light follows the lights traced before it)."""
+    import torch
+    from vulkanhybridraytracer_gb300.hybrid import HybridContext, pass_config
+    wl = _scene(n_lights)
+    ctx = HybridContext(0)
+    try:
+        ctx.set_scene(wl.scene)
+        ctx.build_bvh()
+        cam = wl.scene.camera.rt_camera(w, h, 5.0)
+        planes = ctx.gbuffer(cam, w, h)
+        outs = []
+        for flags, chunk in ((L.HY_FLAG_PIXEL_PARALLEL, 0), (0, 0), (0, 5)):
+            raw = torch.zeros((n_lights, h, w), dtype=torch.uint8, device="cuda")
+            torch.cuda.synchronize()
+            st = ctx.shadow_pass(planes, cam, pass_config(spp, 1, L.HY_RNG_DECORRELATED, 5, flags, queue_chunk=chunk), raw)
+            outs.append((raw, st["shadow_rays"]))
+        for raw, rays in outs[1:]:
+            assert torch.equal(raw, outs[0][0]) and rays == outs[0][1]
+    finally:
+        ctx.close()

@@ -387,7 +387,27 @@ int run_pixels(HyCtx* c, int mode, const PassParams& P0, const HyPassConfig* cfg
     // against 2.28 uncapped (167 registers), 2.03 / 1.91 / 1.86 at 4 / 5 / 6
     P.shade_minb = 8;
     int grid = grid_for(c, mode, count, minb, P.short_stack != 0, (int)P.shade_minb, block);
-    grid = std::max(1, std::min<int>(grid, (int)((P.ntiles * 32ull + block - 1) / block)));
+    P.units = P.whole_tiles = P.ntiles;
+    P.parts = 1;
+    P.part_lights = P.num_lights;
+    if (streams && P.num_lights > 1) {
+        // The launch ends when its last tile does, and a warp may take its last tile
+        // when the others run out of work: the tiles of the last rounds of the resident
+        // warps go out in parts, each a few of the tile's lights.  Many samples per light:
+        // 3 rounds in up to 8 parts (shadow kernel, whole / 1 round / 3 / all tiles: 1080p
+        // 16.51 / 15.85 / 15.84 / 15.91 ms, 512x512 with 8 lights 4.94 / 3.75 / 3.59 / 3.59,
+        // 1277x719 two-level 12.95 / 11.85 / 11.04 / 11.34).  One ray per light: a part sets
+        // its pixels up anew for a few rays, so 1 round in 2 parts (1700x900 0.191 whole,
+        // 0.182; 3 rounds in 8 parts 0.199; 4K with 64 lights 125.2, 125.0).
+        const bool one = mode == MODE_SHADOW_S1 || mode == MODE_SHADOW_ACCUM_S1;
+        const uint32_t rounds = one ? 1 : 3, max_parts = one ? 2 : 8;
+        const uint64_t tail = (uint64_t)rounds * (uint32_t)grid * (uint32_t)(block / 32);
+        P.part_lights = (P.num_lights + max_parts - 1) / max_parts;
+        P.parts = (P.num_lights + P.part_lights - 1) / P.part_lights;
+        P.whole_tiles = P.ntiles - (uint32_t)std::min<uint64_t>(P.ntiles, tail);
+        P.units = P.whole_tiles + (P.ntiles - P.whole_tiles) * P.parts;
+    }
+    grid = std::max(1, std::min<int>(grid, (int)((P.units * 32ull + block - 1) / block)));
     ProfScope prof(c, mode);
     HY_CUDA_TRY(launch_pixels(mode, count, minb, scene_dev(c), P, grid, block, c->stream));
     return HY_OK;

@@ -16,7 +16,8 @@ namespace hy {
 
 // A warp pulls (view, tile) units from the batch's queue and walks each tile
 // light by light (stream_tile) with that view's parameters; REFERENCE-RNG views
-// trace one ray per pixel-light.  ANY_TWO: the batch holds a two-level scene
+// trace one ray per pixel-light (stream_tile_one as a second path in this kernel
+// raised its spills 332 -> 388 B and cost a batch of mixed samples 2.3 %).  ANY_TWO: the batch holds a two-level scene
 // (compiled separately: the second traversal raises the register pressure of
 // the one-level case).  SHORT > 0: the first SHORT stack entries of each lane in
 // dynamic shared memory (SHORT x BLOCK x 8 bytes), entry i of thread t at
@@ -67,22 +68,18 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_shadow_batch_stream(const Batch
         const bool accum = !(P.flags & HY_FLAG_NO_ACCUM) && P.accum_frame > 0;
         const bool reference = P.rng_mode == HY_RNG_REFERENCE;
         const uint32_t tile = unit - P.tile_begin;
-        const bool one = reference || P.spp == 1;  // one ray per pixel and light
-        WalkAreaT<ANY_TWO>& own = sm.scratch[warp].walk;
         if constexpr (ANY_TWO) {  // compiled without a shared stack
             if (S.two_level) {
                 WorldRaySlot w{s_world + threadIdx.x, &sm.scratch[warp].walk.ray[lane]};
-                if (one) stream_tile_one<COUNT, true, 2>(S, P, tile, reference, accum, own, stk, t, w, s, ls, nn, nt);
-                else stream_tile<COUNT, true, 2>(S, P, tile, reference, accum, sm, stk, t, w, s, ls, nn, nt);
+                stream_tile<COUNT, true, 2>(S, P, tile, 0, P.num_lights, reference, accum, sm, stk, t, w, s, ls, nn, nt);
                 continue;
             }
         }
-        auto run = [&](auto stack) {
-            if (one) stream_tile_one<COUNT, false, 2>(S, P, tile, reference, accum, own, stack, t, r, s, ls, nn, nt);
-            else stream_tile<COUNT, false, 2>(S, P, tile, reference, accum, sm, stack, t, r, s, ls, nn, nt);
-        };
-        if constexpr (SHORT > 0) run(SplitStackT<SHORT, BLOCK>{s_stack + threadIdx.x, stk});
-        else run((uint2*)stk);
+        if constexpr (SHORT > 0)
+            stream_tile<COUNT, false, 2>(S, P, tile, 0, P.num_lights, reference, accum, sm,
+                                         SplitStackT<SHORT, BLOCK>{s_stack + threadIdx.x, stk}, t, r, s, ls, nn, nt);
+        else
+            stream_tile<COUNT, false, 2>(S, P, tile, 0, P.num_lights, reference, accum, sm, stk, t, r, s, ls, nn, nt);
     }
     if (COUNT) { ls.nodes += nn; ls.tris += nt; }
     flush_stats(ls, B.stats);

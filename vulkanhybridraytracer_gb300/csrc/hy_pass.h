@@ -30,6 +30,9 @@ struct PassParams {
     float* out_f;
     uint8_t* out_8;
     uint32_t tiles_x, ntiles, chunk;
+    // tile streams: the queue's units are whole_tiles tiles, then parts units per tile, each
+    // of part_lights lights
+    uint32_t units, whole_tiles, parts, part_lights;
     uint32_t blur_w, blur_h; // texels the blur dispatch covers
     uint32_t group;          // lanes per pixel-light in the sample-parallel shadow kernel
     uint32_t inner;          // node visits per scheduling round of that kernel (>= 1)

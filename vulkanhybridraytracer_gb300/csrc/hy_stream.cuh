@@ -362,13 +362,19 @@ __device__ __forceinline__ void stream_pixel(const SceneDev& S, const PassParams
     s.in_blur = x < P.blur_w && y < P.blur_h;
 }
 
+// whether a light's shadow rays are traced for the pixel (shadowRaygen.rgen:43-63)
+__device__ __forceinline__ bool light_traced(const HyLight& lt, const ShadowLane& s) {
+    const LightGeo lg = light_geo(lt, s.position, s.N);
+    return s.smode != 4 && lg.NdotL > 0.f && lg.dist < lg.maxd;
+}
+
 // ---------------------------------------------------------------------------------
-// One 8x4 tile of a view, light by light.  ACC: 0 raw shadow images, 1 the
+// Lights light0 .. light1 - 1 of one 8x4 tile of a view, light by light.  ACC: 0 raw shadow images, 1 the
 // running mean into the history, 2 either (accum) at run time.  reference:
 // REFERENCE RNG (one ray per pixel-light from the pixel's seed, by value).
 template <bool COUNT, bool TWO, int ACC, class Stack, class Slots, class RW>
-__device__ __forceinline__ void stream_tile(const SceneDev& S, const PassParams& P, uint32_t tile, bool reference,
-                                            bool accum, Slots& sm, Stack stk, Trav& t, RW& r,
+__device__ __forceinline__ void stream_tile(const SceneDev& S, const PassParams& P, uint32_t tile, uint32_t light0,
+                                            uint32_t light1, bool reference, bool accum, Slots& sm, Stack stk, Trav& t, RW& r,
                                             ShadowLane& s, LaneStats& ls, uint32_t& nn, uint32_t& nt) {
     const uint32_t lane = threadIdx.x & 31, wb = threadIdx.x & ~31u;
     const size_t plane = (size_t)P.W * P.H;
@@ -383,8 +389,10 @@ __device__ __forceinline__ void stream_tile(const SceneDev& S, const PassParams&
     if (present) {
         stream_pixel(S, P, x, y, s);
         seed0 = s.seed;
+#pragma unroll 1
+        for (uint32_t l = 0; l < light0; l++) rays_before += light_traced(S.lights[l], s) ? spp : 0u;
     }
-    for (uint32_t l = 0; l < P.num_lights; l++) {
+    for (uint32_t l = light0; l < light1; l++) {
         // ---- light l for this lane's pixel ----
         bool traced = false;
         s.light = l;
@@ -426,9 +434,10 @@ __device__ __forceinline__ void stream_tile(const SceneDev& S, const PassParams&
 // Each pixel's lights keep their order, so the RNG states are the sequential loop's.
 constexpr uint32_t kSetupLanes = 16, kLightDrift = 8;
 template <bool COUNT, bool TWO, int ACC, class Area, class Stack, class RW>
-__device__ __forceinline__ void stream_tile_one(const SceneDev& S, const PassParams& P, uint32_t tile, bool reference,
-                                                bool accum, Area& w, Stack stk, Trav& t, RW& r, ShadowLane& s,
-                                                LaneStats& ls, uint32_t& nn, uint32_t& nt) {
+__device__ __forceinline__ void stream_tile_one(const SceneDev& S, const PassParams& P, uint32_t tile,
+                                                uint32_t light0, uint32_t light1, bool reference, bool accum, Area& w,
+                                                Stack stk, Trav& t, RW& r, ShadowLane& s, LaneStats& ls, uint32_t& nn,
+                                                uint32_t& nt) {
     const uint32_t lane = threadIdx.x & 31;
     const size_t plane = (size_t)P.W * P.H;
     const uint32_t x = (tile % P.tiles_x) * 8 + (lane & 7), y = (tile / P.tiles_x) * 4 + (lane >> 3);
@@ -437,10 +446,13 @@ __device__ __forceinline__ void stream_tile_one(const SceneDev& S, const PassPar
         if (ACC == 0 || (ACC == 2 && !accum)) shadow_finalize<false>(P, s, plane, v);
         else shadow_finalize<true>(P, s, plane, v);
     };
-    uint32_t next = P.num_lights;  // the pixel's next light to set up
+    uint32_t next = light1;  // the pixel's next light to set up
     if (x < P.W && y < P.H) {
         stream_pixel(S, P, x, y, s);
-        next = 0;
+        next = light0;
+#pragma unroll 1
+        for (uint32_t l = 0; l < light0 && !reference; l++)
+            if (light_traced(S.lights[l], s)) s.seed = lcg_jump_even(s.seed, 1);
     }
     bool live = false, ready = false;       // walking a ray; a prepared one waits
     uint32_t light = 0, ready_light = 0;    // their lights
@@ -450,10 +462,10 @@ __device__ __forceinline__ void stream_tile_one(const SceneDev& S, const PassPar
     if (lane == 0) w.npairs = 0;
     __syncwarp();
     for (;;) {
-        const uint32_t starved = __ballot_sync(0xffffffffu, !live && !ready && next < P.num_lights);
+        const uint32_t starved = __ballot_sync(0xffffffffu, !live && !ready && next < light1);
         if (starved && ((uint32_t)__popc(starved) >= kSetupLanes || __ballot_sync(0xffffffffu, live || ready) == 0)) {
             const uint32_t last = __reduce_min_sync(0xffffffffu, live ? light : (ready ? ready_light : next));
-            while (!ready && next < P.num_lights && next - last <= kLightDrift) {
+            while (!ready && next < light1 && next - last <= kLightDrift) {
                 const uint32_t l = next++;
                 const HyLight& lt = S.lights[l];
                 const LightGeo lg = light_geo(lt, s.position, s.N);
@@ -483,7 +495,7 @@ __device__ __forceinline__ void stream_tile_one(const SceneDev& S, const PassPar
             ready = false;
         }
         if (__ballot_sync(0xffffffffu, live) == 0) {
-            if (__ballot_sync(0xffffffffu, next < P.num_lights) == 0) break;
+            if (__ballot_sync(0xffffffffu, next < light1) == 0) break;
             continue;
         }
         const RoundResult res = stream_round<COUNT, TWO>(S, P, w, live, stk, t, r, nn, nt);

@@ -55,24 +55,33 @@ __global__ void __launch_bounds__(128, MINB) k_shadow_stream(const SceneDev S, c
         else r.ray = &sm.scratch[threadIdx.x >> 5].walk.ray[lane];
     }
     uint32_t chunk_cur = 0, chunk_end = 0, nn = 0, nt = 0;
+    const bool reference = P.rng_mode == HY_RNG_REFERENCE;
     for (;;) {
         if (chunk_cur == chunk_end) {
             uint32_t t0 = 0;
             if (lane == 0) t0 = atomicAdd(P.queue, P.chunk);
             t0 = __shfl_sync(0xffffffffu, t0, 0);
-            if (t0 >= P.ntiles) break;
+            if (t0 >= P.units) break;
             chunk_cur = t0;
-            chunk_end = min(t0 + P.chunk, P.ntiles);
+            chunk_end = min(t0 + P.chunk, P.units);
         }
-        const bool reference = P.rng_mode == HY_RNG_REFERENCE;
+        // a unit: a whole tile, or (the last ones) one part of a tile's lights
+        const uint32_t unit = chunk_cur++;
+        uint32_t tile = unit, l0 = 0, l1 = P.num_lights;
+        if (unit >= P.whole_tiles) {
+            const uint32_t u = unit - P.whole_tiles, part = u % P.parts;
+            tile = P.whole_tiles + u / P.parts;
+            l0 = part * P.part_lights;
+            l1 = min(l0 + P.part_lights, P.num_lights);
+        }
         if constexpr (ONE)
-            stream_tile_one<COUNT, TWO, ACCUM ? 1 : 0>(S, P, chunk_cur++, reference, ACCUM, sm.warp[threadIdx.x >> 5],
+            stream_tile_one<COUNT, TWO, ACCUM ? 1 : 0>(S, P, tile, l0, l1, reference, ACCUM, sm.warp[threadIdx.x >> 5],
                                                        stk, t, r, s, ls, nn, nt);
         else if constexpr (SHORT)
-            stream_tile<COUNT, TWO, ACCUM ? 1 : 0>(S, P, chunk_cur++, reference, ACCUM, sm,
+            stream_tile<COUNT, TWO, ACCUM ? 1 : 0>(S, P, tile, l0, l1, reference, ACCUM, sm,
                                                    SplitStack{s_stack + threadIdx.x, stk}, t, r, s, ls, nn, nt);
         else
-            stream_tile<COUNT, TWO, ACCUM ? 1 : 0>(S, P, chunk_cur++, reference, ACCUM, sm, stk, t, r, s, ls, nn, nt);
+            stream_tile<COUNT, TWO, ACCUM ? 1 : 0>(S, P, tile, l0, l1, reference, ACCUM, sm, stk, t, r, s, ls, nn, nt);
     }
     if (COUNT) { ls.nodes += nn; ls.tris += nt; }
     flush_stats(ls, P.stats);
