@@ -762,9 +762,12 @@ int hy_trace_rays(HyCtx* c, const HyRay* rays, uint32_t n, int any_hit, HyHit* h
     int rc = reset_counters(c);
     if (rc) return rc;
     bool count = st != nullptr;
-    int grid = std::max(1, std::min<int>(c->num_sms * 16, (int)((n + 127) / 128)));
-    HY_CUDA_TRY(launch_trace(scene_dev(c), rays, n, any_hit != 0, count, hits, dev_stats(c), dev_status(c), grid,
-                             c->stream));
+    // queries that report no counts: 8 resident blocks per SM on the closest-hit queue
+    // (which loads and stores 16 bytes at a time)
+    const bool queued = !count && any_hit == 0 && n <= 0xfff00000u && ((uintptr_t)rays | (uintptr_t)hits) % 16 == 0;
+    int grid = std::max(1, std::min<int>(c->num_sms * (queued ? 8 : 16), (int)((n + 127) / 128)));
+    HY_CUDA_TRY(launch_trace(scene_dev(c), rays, n, any_hit != 0, count, hits, dev_stats(c), dev_status(c),
+                             queued ? dev_queue(c, WQ_MISC) : nullptr, grid, c->stream));
     return finish_call(c, st, true);
 }
 

@@ -24,6 +24,8 @@
 // sized to the resident-block capacity of the GPU.
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "hy_device.cuh"
 #include "hy_pass.h"
 #include "hy_shade.cuh"
@@ -496,9 +498,11 @@ __global__ void k_accumulate(const AccumParams A) {
     }
 }
 
-// generic ray queries (32 B ray in, 16 B hit out)
+// generic ray queries (32 B ray in, 16 B hit out), a thread per ray: any-hit ones (8
+// resident blocks: 2M incoherent rays 592 -> 461 us, the call), counting ones, and
+// buffers that are not 16-byte aligned
 template <bool ANY, bool COUNT>
-__global__ void __launch_bounds__(128) k_trace(const SceneDev S, const HyRay* __restrict__ rays, uint32_t n,
+__global__ void __launch_bounds__(128, 8) k_trace(const SceneDev S, const HyRay* __restrict__ rays, uint32_t n,
                                                HyHit* __restrict__ hits, unsigned long long* stats, uint32_t* status) {
     LaneStats ls;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i - threadIdx.x < n; i += gridDim.x * blockDim.x) {
@@ -520,6 +524,71 @@ __global__ void __launch_bounds__(128) k_trace(const SceneDev S, const HyRay* __
     flush_stats(ls, stats);
 }
 
+// Closest-hit queries: persistent warps whose idle lanes take the next rays of the
+// queue, kTraceRefill or more at a time, walking with their triangles tested together
+// (closest_round).  A thread per ray waited for the longest walk of its warp and tested
+// triangles on one or two lanes: 262k / 2M incoherent rays over 1.5M triangles, the call
+// 164 / 904 -> 131 / 415 us (refills of 1 / 4 / 8 / 16 / 24 lanes: 425 / 423 / 425 / 451
+// / 511).
+constexpr uint32_t kTraceRefill = 4;
+template <bool TWO>
+__global__ void __launch_bounds__(128, 8) k_trace_closest(const SceneDev S, const HyRay* __restrict__ rays, uint32_t n,
+                                                          HyHit* __restrict__ hits, uint32_t* queue, uint32_t* status) {
+    __shared__ ClosestAreaT<TWO> s_area[4];
+    __shared__ float s_world[TWO ? 6 * 128 : 1];
+    ClosestAreaT<TWO>& w = s_area[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31;
+    uint2 stk[kStackMax];
+    Trav t;
+    std::conditional_t<TWO, WorldRaySlot, RayPre> r{};
+    if constexpr (TWO) {
+        r.p = s_world + threadIdx.x;
+        r.ray = &w.ray[lane];
+    }
+    bool live = false, more = true;
+    uint32_t i = 0;
+    float tmin = 0.f;
+    if (lane == 0) w.npairs = 0;
+    __syncwarp();
+    for (;;) {
+        const uint32_t idle = __ballot_sync(0xffffffffu, !live);
+        if (more && ((uint32_t)__popc(idle) >= kTraceRefill || idle == 0xffffffffu)) {
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(queue, (uint32_t)__popc(idle));
+            base = __shfl_sync(0xffffffffu, base, 0);
+            more = base + (uint32_t)__popc(idle) < n;
+            const uint32_t mine = base + (uint32_t)__popc(idle & ((1u << lane) - 1u));
+            if (!live && mine < n) {
+                i = mine;
+                const float4 a = __ldg((const float4*)(rays + i)), b = __ldg((const float4*)(rays + i) + 1);
+                tmin = a.w;
+                // an empty interval enters no box (the walk's box test takes tmin <= tmax for granted)
+                const float tmax = tmin > __fmul_rn(b.w, kBoxSlack) ? -INFINITY : b.w;
+                closest_start<TWO>(w, t, r, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), tmin, tmax);
+                live = true;
+            }
+        }
+        if (__ballot_sync(0xffffffffu, live) == 0) {
+            if (!more) break;
+            continue;
+        }
+        uint32_t limits = 0;
+        const bool over = closest_round<TWO>(S, w, live, tmin, (uint2*)stk, t, r, limits, status);
+        if (live && over) {
+            if (limits) {  // a limit ran out: the plain walk decides
+                const float4 d = w.ray[lane];
+                const HyRay& q = rays[i];
+                const float tmax = q.tmin > __fmul_rn(q.tmax, kBoxSlack) ? -INFINITY : q.tmax;
+                t.h = traverse_again<TWO>(S, mk(q.org[0], q.org[1], q.org[2]), mk(d.x, d.y, d.z), q.tmin, tmax, status);
+            }
+            const bool hit = t.h.id != HY_NO_HIT;
+            reinterpret_cast<float4*>(hits)[i] = make_float4(hit ? t.h.t : 0.f, __uint_as_float(t.h.id),
+                                                             hit ? t.h.b1 : 0.f, hit ? t.h.b2 : 0.f);
+            live = false;
+        }
+    }
+}
+
 // primary-ray G-buffer (raygen.rgen:29-40 camera, geometry_shader.frag:54-76 encoding)
 __device__ __forceinline__ f3 mat_vec3(const float* m, float x, float y, float z, float w) {
     float r[3];
@@ -534,8 +603,13 @@ __device__ __forceinline__ f3 mat_vec3(const float* m, float x, float y, float z
     return mk(r[0], r[1], r[2]);
 }
 
-__global__ void __launch_bounds__(128) k_gbuffer(const SceneDev S, const GbufParams G) {
-    uint32_t x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
+// A warp per 8x4 tile; compiled per structure level, each with one copy of the walk, for
+// 8 resident blocks (1080p, the call: 16x2 texels a warp, 94 registers 458 us; 8x4 tiles
+// at 1 / 6 / 8 / 10 / 12 blocks 434 / 409 / 385 / 394 / 409).
+template <bool TWO>
+__global__ void __launch_bounds__(128, 8) k_gbuffer(const SceneDev S, const GbufParams G) {
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t x = blockIdx.x * 16 + (warp & 1) * 8 + (lane & 7), y = blockIdx.y * 8 + (warp >> 1) * 4 + (lane >> 3);
     if (x >= G.W || y >= G.H) return;
     size_t i = (size_t)y * G.W + x;
     float ux = __fdiv_rn(__fadd_rn((float)x, 0.5f), (float)G.W), uy = __fdiv_rn(__fadd_rn((float)y, 0.5f), (float)G.H);
@@ -546,7 +620,7 @@ __global__ void __launch_bounds__(128) k_gbuffer(const SceneDev S, const GbufPar
     f3 dir = mat_vec3(G.inv_view, tn.x, tn.y, tn.z, 0.f);
     f3 o = add_rn(org, scale_rn(dir, 1e-2f));
     LaneStats ls;
-    Hit h = trace<false, false>(S, o, dir, 0.001f, 10000.0f, ls, G.status);
+    const Hit h = trace<false, false, TWO ? 2 : 1>(S, o, dir, 0.001f, 10000.0f, ls, G.status);
     float4* p0 = (float4*)G.planes[0]; float4* p1 = (float4*)G.planes[1]; float4* p2 = (float4*)G.planes[2];
     float2* p3 = (float2*)G.planes[3]; float4* p4 = (float4*)G.planes[4]; float4* p5 = (float4*)G.planes[5];
     if (h.id == HY_NO_HIT) {
@@ -1059,21 +1133,24 @@ cudaError_t launch_accumulate(const AccumParams& A, cudaStream_t s) {
 }
 
 cudaError_t launch_trace(const SceneDev& S, const HyRay* rays, uint32_t n, bool any, bool count, HyHit* hits,
-                         unsigned long long* stats, uint32_t* status, int grid, cudaStream_t s) {
+                         unsigned long long* stats, uint32_t* status, uint32_t* queue, int grid, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
     if (any) {
         if (count) k_trace<true, true><<<grid, 128, 0, s>>>(S, rays, n, hits, stats, status);
         else k_trace<true, false><<<grid, 128, 0, s>>>(S, rays, n, hits, stats, status);
     } else {
         if (count) k_trace<false, true><<<grid, 128, 0, s>>>(S, rays, n, hits, stats, status);
-        else k_trace<false, false><<<grid, 128, 0, s>>>(S, rays, n, hits, stats, status);
+        else if (!queue) k_trace<false, false><<<grid, 128, 0, s>>>(S, rays, n, hits, stats, status);
+        else if (S.two_level) k_trace_closest<true><<<grid, 128, 0, s>>>(S, rays, n, hits, queue, status);
+        else k_trace_closest<false><<<grid, 128, 0, s>>>(S, rays, n, hits, queue, status);
     }
     return cudaGetLastError();
 }
 
 cudaError_t launch_gbuffer(const SceneDev& S, const GbufParams& G, cudaStream_t s) {
-    dim3 b(16, 8), g((G.W + 15) / 16, (G.H + 7) / 8);
-    k_gbuffer<<<g, b, 0, s>>>(S, G);
+    dim3 g((G.W + 15) / 16, (G.H + 7) / 8);
+    if (S.two_level) k_gbuffer<true><<<g, 128, 0, s>>>(S, G);
+    else k_gbuffer<false><<<g, 128, 0, s>>>(S, G);
     return cudaGetLastError();
 }
 

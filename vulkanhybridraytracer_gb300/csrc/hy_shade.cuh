@@ -42,18 +42,28 @@ __device__ __forceinline__ Hit trace(const SceneDev& S, f3 o, f3 d, float tmin, 
     return h;
 }
 
-// equirect NEAREST / REPEAT lookup of an RGBA8 map
-__device__ __forceinline__ f3 env_lookup(const uchar4* px, uint32_t w, uint32_t h, float u, float v) {
+// a ray by itself, out of line: for the rays whose walk ran into a limit
+template <bool TWO>
+__device__ __noinline__ Hit traverse_again(const SceneDev& S, f3 o, f3 d, float tmin, float tmax, uint32_t* status) {
+    uint32_t nn = 0, nt = 0;
+    return traverse<false, false, TWO>(S, ray_pre(o, d), tmin, tmax, &nn, &nt, status);
+}
+
+// equirect NEAREST / REPEAT lookup of an RGBA8 map.  One copy for all callers (the
+// shade kernel waits on instruction fetches), and 32-bit remainders: the
+// texel coordinates are clamped to +-1e9.
+__device__ __forceinline__ uint32_t wrap_texel(int i, uint32_t n) {
+    if (i >= 0) return (uint32_t)i % n;
+    return n - 1u - (uint32_t)(-1 - i) % n;  // i mod n of a negative i
+}
+static __device__ __noinline__ f3 env_lookup(const uchar4* px, uint32_t w, uint32_t h, float u, float v) {
     if (w == 0 || h == 0) return mk(0.f, 0.f, 0.f);
     if (!(u == u)) u = 0.f;
     if (!(v == v)) v = 0.f;
     float fx = floorf(u * (float)w), fy = floorf(v * (float)h);
     fx = fminf(fmaxf(fx, -1e9f), 1e9f);
     fy = fminf(fmaxf(fy, -1e9f), 1e9f);
-    long long ix = (long long)fx % (long long)w, iy = (long long)fy % (long long)h;
-    if (ix < 0) ix += w;
-    if (iy < 0) iy += h;
-    uchar4 c = px[(size_t)iy * w + (size_t)ix];
+    const uchar4 c = px[(size_t)wrap_texel((int)fy, h) * w + wrap_texel((int)fx, w)];
     return mk(__fdiv_rn((float)c.x, 255.f), __fdiv_rn((float)c.y, 255.f), __fdiv_rn((float)c.z, 255.f));
 }
 __device__ __forceinline__ f3 irradiance_at(const SceneDev& S, f3 N) {

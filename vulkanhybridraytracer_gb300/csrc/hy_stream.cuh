@@ -211,6 +211,120 @@ __device__ __forceinline__ RoundResult stream_round(const SceneDev& S, const Pas
     return res;
 }
 
+// ---- closest-hit walks of a warp, their triangles tested together ------------------
+// (k_trace_closest.  For the G-buffer's primary rays, whose plain walks agree already,
+// the later shrinking interval cost more than the tests: 1080p, the call 458 -> 543 us.)
+// As stream_round, for closest-hit rays: pairs are collected over a round, each
+// tested by one lane against its owner's interval as it was when the round began;
+// hits meet in the owner's 64-bit key (distance, id; the lower id on equal
+// distances), and the pair whose key is left hands its distance and barycentrics
+// over.  The closest hit does not depend on the order of visits or on how early the
+// interval shrinks, so it is the plain walk's, bit for bit; a ray may make a few more
+// node visits.  A ray that runs into a limit is walked anew by itself (plain), so
+// that the limit holds for the plain walk's visits.
+template <bool TWO>
+struct ClosestAreaT : WalkAreaT<TWO> {  // ray[].w: tmin
+    unsigned long long key[32];         // per owner: (order-preserving distance bits, id)
+    float4 best[32];                    // its distance and barycentrics
+};
+
+// distances as unsigned keys in order (-0 and +0 one key)
+__device__ __forceinline__ uint32_t distance_key(float t) {
+    const uint32_t b = __float_as_uint(__fadd_rn(t, 0.f));
+    return b & 0x80000000u ? ~b : b | 0x80000000u;
+}
+
+template <bool TWO, class RW>
+__device__ __forceinline__ void closest_start(ClosestAreaT<TWO>& w, Trav& t, RW& r, f3 o, f3 d, float tmin, float tmax) {
+    const uint32_t lane = threadIdx.x & 31;
+    w.ray[lane] = make_float4(d.x, d.y, d.z, tmin);
+    w.key[lane] = ~0ull;
+    trav_init(t, world_set(r, o, d), tmax);
+}
+
+// One round; live lanes get whether their walk is over (t.h then holds the hit).
+// The interval shrinks only at the end of a round, the tests fill their lanes only
+// over several visits: 2M incoherent queries over 1.5M triangles at 1 / 2 / 3 / 4 / 6
+// visits 525 / 457 / 425 / 415 / 438 us (a thread per ray, tests at once: 904 us).
+constexpr uint32_t kClosestVisits = 4;
+template <bool TWO, class Stack, class RW>
+__device__ __forceinline__ bool closest_round(const SceneDev& S, ClosestAreaT<TWO>& w, bool live, float tmin,
+                                              Stack stk, Trav& t, RW& r, uint32_t& limits, uint32_t* status) {
+    const uint32_t lane = threadIdx.x & 31;
+    bool over = false;
+    if (live) {
+        uint32_t none = 0;
+#pragma unroll 1
+        for (uint32_t it = 0; it < kClosestVisits; it++) {
+            if (trav_node<false, false, TWO>(S, r, tmin, t, stk, none, DeferredStatus{limits})) {
+                over = true;
+                break;
+            }
+            if (t.pend_bits) {
+                pairs_push<TWO>(w, t);
+                if (t.pend_bits) break;
+            }
+        }
+    }
+    for (;;) {
+        __syncwarp();
+        const uint32_t np = min(w.npairs, kPairs);
+        if (np == 0) break;
+        for (uint32_t b = 0; b < np; b += 32) {
+            const uint32_t i = b + lane;
+            const uint32_t owner = i < np ? (uint32_t)w.owner[i] : lane;
+            const float tmax = __shfl_sync(0xffffffffu, t.tmax, owner);
+            f3 o;
+            if constexpr (TWO) {
+                const int d = (int)owner - (int)lane;
+                o = mk(r.p[d], r.p[d + 128], r.p[d + 256]);
+            } else {
+                o = mk(__shfl_sync(0xffffffffu, r.o.x, owner), __shfl_sync(0xffffffffu, r.o.y, owner),
+                       __shfl_sync(0xffffffffu, r.o.z, owner));
+            }
+            unsigned long long key = ~0ull;
+            float tt = 0.f, b1 = 0.f, b2 = 0.f;
+            if (i < np) {
+                const uint32_t rec = w.rec[i];
+                if (rec < S.num_tris) {
+                    const float4 ray = w.ray[owner];
+                    f3 dir = mk(ray.x, ray.y, ray.z);
+                    uint32_t id0 = 0;
+                    if constexpr (TWO) {
+                        const float4* I = S.inst + (size_t)w.inst[i] * 4;
+                        const float4 r0 = __ldg(I), r1 = __ldg(I + 1), r2 = __ldg(I + 2);
+                        id0 = __float_as_uint(__ldg(I + 3).y);
+                        o = xform_point(r0, r1, r2, o);
+                        dir = xform_dir(r0, r1, r2, dir);
+                    }
+                    const float4* tp = S.tris + (size_t)rec * 3;
+                    const float4 v0 = __ldg(tp);
+                    if (tri_test(ray_pre(o, dir), v0, __ldg(tp + 1), __ldg(tp + 2), ray.w, tmax, tt, b1, b2)) {
+                        key = ((unsigned long long)distance_key(tt) << 32) | (id0 + __float_as_uint(v0.w));
+                        atomicMin(&w.key[owner], key);
+                    }
+                } else {
+                    atomicOr(status, HY_STATUS_BAD_INDEX);
+                }
+            }
+            __syncwarp();
+            if (key != ~0ull && w.key[owner] == key) w.best[owner] = make_float4(tt, b1, b2, 0.f);
+            __syncwarp();
+        }
+        if (lane == 0) w.npairs = 0;
+        const unsigned long long key = w.key[lane];
+        if (live && key != ~0ull) {
+            const float4 h = w.best[lane];
+            t.h = Hit{h.x, (uint32_t)key, h.y, h.z};
+            t.tmax = h.x;
+        }
+        __syncwarp();
+        if (__ballot_sync(0xffffffffu, live && t.pend_bits != 0) == 0) break;
+        if (live && t.pend_bits) pairs_push<TWO>(w, t);
+    }
+    return over;
+}
+
 // The warp's items of one light (every lane calls it, after all lanes have
 // published): sample k of a pixel starts from its first state advanced 2k LCG
 // steps (sampleDisk's two draws per sample), its ray from position +
