@@ -64,7 +64,11 @@ static_assert(sizeof(SahRange) == 40, "SahRange layout");
 struct SahChunk { uint32_t node, start, end, first; };  // range slot, [start, end), the range's first chunk
 struct SahSplit { int axis, q; uint32_t m, child[2]; };  // child: 0 none, 1 << 30 | next-level slot, 2 << 30 | small slot
 
-enum { CTR_NEXT = 0, CTR_SMALL = 1, CTR_ROOT = 2, CTR_ERR = 3 };
+enum { CTR_NEXT = 0, CTR_SMALL = 1, CTR_ROOT = 2, CTR_ERR = 3, CTR_TINY = 4, CTR_COUNT };
+
+// ranges of up to kTiny triangles: whole subtrees for one thread each (k_sah_tiny)
+constexpr uint32_t kTiny = 8;
+struct SahTiny { uint32_t f, l, parent, side; };
 
 __device__ __forceinline__ int okey(float x) {
     const int b = __float_as_int(x);
@@ -466,7 +470,8 @@ constexpr int kSmallWarps = 4;
 __global__ void __launch_bounds__(32 * kSmallWarps) k_sah_small(const SahRange* __restrict__ tasks, uint32_t ntask,
                                                                 uint32_t n, const float4* __restrict__ cen,
                                                                 const float* __restrict__ box, uint32_t* ord,
-                                                                uint32_t* ord2, uint32_t* __restrict__ bvh2,
+                                                                uint32_t* ord2, SahTiny* __restrict__ tiny,
+                                                                uint32_t* __restrict__ bvh2,
                                                                 uint32_t* __restrict__ parent,
                                                                 uint32_t* __restrict__ ctr) {
     __shared__ int s_bins[kSmallWarps][kNodeBinWords];
@@ -477,6 +482,13 @@ __global__ void __launch_bounds__(32 * kSmallWarps) k_sah_small(const SahRange* 
     int* bins = s_bins[w];
     SahRange cur = tasks[task];
     int sp = 0;
+    auto queue_tiny = [&](uint32_t f, uint32_t l, uint32_t par, uint32_t side) {
+        if (lane == 0) tiny[atomicAdd(ctr + CTR_TINY, 1u)] = SahTiny{f, l, par, side};
+    };
+    if (cur.l - cur.f + 1 <= kTiny) {
+        queue_tiny(cur.f, cur.l, cur.parent, cur.side);
+        return;
+    }
     for (;;) {
         const uint32_t f = cur.f, l = cur.l, c = l - f + 1;
         const Axes x = axes_of(cur.ck);
@@ -543,7 +555,10 @@ __global__ void __launch_bounds__(32 * kSmallWarps) k_sah_small(const SahRange* 
         keys_warp(kr);
         const uint32_t id = m - 1;
         if (lane == 0) write_node(id, f, l, m, cur.parent, cur.side, n, bvh2, parent, ctr);
-        const bool li = m - f >= 2, ri = l - m + 1 >= 2;
+        const uint32_t nleft = m - f, nright = l - m + 1;
+        if (nleft >= 2 && nleft <= kTiny) queue_tiny(f, m - 1, id, 0);
+        if (nright >= 2 && nright <= kTiny) queue_tiny(m, l, id, 1);
+        const bool li = nleft > kTiny, ri = nright > kTiny;
         SahRange L, R;
         L.f = f; L.l = m - 1; L.parent = id; L.side = 0;
         R.f = m; R.l = l; R.parent = id; R.side = 1;
@@ -568,6 +583,100 @@ __global__ void __launch_bounds__(32 * kSmallWarps) k_sah_small(const SahRange* 
             cur = s_stack[w][--sp];
         }
         __syncwarp();
+    }
+}
+
+// ---- one thread per range of 2 .. kTiny triangles ------------------------------
+// Nine of ten internal nodes lie in such subtrees, and a warp with bins per range
+// spent about 2,000 instructions on each.  Here the triangles sit in the thread's
+// local array, their order in the nibbles of one word, and only the splits after an
+// occupied bin are tried: any other split parts the range like the one after the
+// last occupied bin before it, which comes first and so wins.  The same cost
+// expression, tie rule and stable partition, so the same tree.
+__global__ void __launch_bounds__(128) k_sah_tiny(const SahTiny* __restrict__ tasks, uint32_t n,
+                                                  const float4* __restrict__ cen, const float* __restrict__ box,
+                                                  uint32_t* __restrict__ ord, uint32_t* __restrict__ bvh2,
+                                                  uint32_t* __restrict__ parent, uint32_t* __restrict__ ctr) {
+    const uint32_t ntask = ctr[CTR_TINY];
+    for (uint32_t task = blockIdx.x * blockDim.x + threadIdx.x; task < ntask; task += gridDim.x * blockDim.x) {
+        const SahTiny T = tasks[task];
+        const uint32_t cnt = T.l - T.f + 1;
+        uint32_t tri[kTiny];
+        float ce[kTiny][3];
+        int bx[kTiny][6];
+        for (uint32_t k = 0; k < cnt; k++) {
+            tri[k] = ord[T.f + k];
+            const float4 c = cen[tri[k]];
+            ce[k][0] = c.x; ce[k][1] = c.y; ce[k][2] = c.z;
+            const float* b = box + (size_t)tri[k] * 6;
+            for (int j = 0; j < 6; j++) bx[k][j] = okey(b[j]);
+        }
+        uint32_t order = 0x76543210u;  // nibble k: the triangle at position k
+        uint32_t stack[kTiny], par[kTiny];  // first | count << 4 | side << 8; parent node
+        int sp = 1;
+        stack[0] = cnt << 4 | T.side << 8;
+        par[0] = T.parent;
+        while (sp > 0) {
+            sp--;
+            const uint32_t s = stack[sp] & 15u, c = (stack[sp] >> 4) & 15u, side = stack[sp] >> 8, up = par[sp];
+            int ck[6];
+            keys_init(ck);
+            for (uint32_t k = 0; k < c; k++) {
+                const float* p = ce[(order >> (4 * (s + k))) & 15u];
+                keys_add(ck, make_float4(p[0], p[1], p[2], 0.f));
+            }
+            const Axes x = axes_of(ck);
+            unsigned long long best = ~0ull, best_bins = 0;
+            for (int a = 0; a < 3; a++) {
+                if (!x.ok[a]) continue;
+                unsigned long long bins = 0;  // byte k: the bin of the triangle at position s + k
+                for (uint32_t k = 0; k < c; k++)
+                    bins |= (unsigned long long)sah_bin(ce[(order >> (4 * (s + k))) & 15u][a], x.lo[a], x.scale[a])
+                            << (8 * k);
+                for (uint32_t i = 0; i < c; i++) {
+                    const uint32_t q = (uint32_t)(bins >> (8 * i)) & 0xffu;
+                    int llo[3] = {INT_MAX, INT_MAX, INT_MAX}, lhi[3] = {INT_MIN, INT_MIN, INT_MIN};
+                    int rlo[3] = {INT_MAX, INT_MAX, INT_MAX}, rhi[3] = {INT_MIN, INT_MIN, INT_MIN};
+                    uint32_t nl = 0;
+                    for (uint32_t k = 0; k < c; k++) {
+                        const int* b = bx[(order >> (4 * (s + k))) & 15u];
+                        if (((uint32_t)(bins >> (8 * k)) & 0xffu) <= q) {
+                            nl++;
+#pragma unroll
+                            for (int j = 0; j < 3; j++) { llo[j] = min(llo[j], b[j]); lhi[j] = max(lhi[j], b[3 + j]); }
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 3; j++) { rlo[j] = min(rlo[j], b[j]); rhi[j] = max(rhi[j], b[3 + j]); }
+                        }
+                    }
+                    if (nl == c) continue;
+                    const float t1 = __fmul_rn(area_keys(llo, lhi), __uint2float_rn(nl));
+                    const float t2 = __fmul_rn(area_keys(rlo, rhi), __uint2float_rn(c - nl));
+                    const float cost = __fadd_rn(__fadd_rn(t1, t2), 0.f);
+                    if (!(cost < INFINITY)) continue;
+                    const unsigned long long key = ((unsigned long long)__float_as_uint(cost) << 32) | (uint32_t)(a * kBins + q);
+                    if (key < best) { best = key; best_bins = bins; }
+                }
+            }
+            uint32_t nl = c / 2;
+            if (best != ~0ull) {
+                const uint32_t q = (uint32_t)best % kBins;
+                uint32_t left = 0, right = 0, nr = 0;
+                nl = 0;
+                for (uint32_t k = 0; k < c; k++) {
+                    const uint32_t who = (order >> (4 * (s + k))) & 15u;
+                    if (((uint32_t)(best_bins >> (8 * k)) & 0xffu) <= q) left |= who << (4 * nl++);
+                    else right |= who << (4 * nr++);
+                }
+                const uint32_t mask = (c == 8 ? 0xffffffffu : (1u << (4 * c)) - 1u) << (4 * s);
+                order = (order & ~mask) | ((left | right << (4 * nl)) << (4 * s));
+            }
+            const uint32_t f = T.f + s, m = f + nl, id = m - 1;
+            write_node(id, f, f + c - 1, m, up, side, n, bvh2, parent, ctr);
+            if (nl >= 2) { stack[sp] = s | nl << 4; par[sp++] = id; }
+            if (c - nl >= 2) { stack[sp] = (s + nl) | (c - nl) << 4 | 1u << 8; par[sp++] = id; }
+        }
+        for (uint32_t k = 0; k < cnt; k++) ord[T.f + k] = tri[(order >> (4 * k)) & 15u];
     }
 }
 
@@ -598,10 +707,14 @@ int sah_tree_impl(HyCtx* c, uint32_t n, uint32_t* ord, uint32_t* ord2, uint32_t*
         (rc = ctx_alloc(c, c->sah_chunks, (size_t)chunkcap * sizeof(SahChunk))) ||
         (rc = ctx_alloc(c, c->sah_first, (size_t)bigcap * 4)) ||
         (rc = ctx_alloc(c, c->sah_ccnt, (size_t)chunkcap * 3 * kBins * 4)) ||
-        (rc = ctx_alloc(c, c->sah_coff, (size_t)chunkcap * 4)) || (rc = ctx_alloc(c, c->sah_ctr, 16)))
+        (rc = ctx_alloc(c, c->sah_coff, (size_t)chunkcap * 4)) || (rc = ctx_alloc(c, c->sah_ctr, CTR_COUNT * 4)))
         return rc;
     uint32_t* ctr = c->sah_ctr.as<uint32_t>();
-    HY_CUDA_TRY(cudaMemsetAsync(ctr, 0, 16, s));
+    // at most n / 2 ranges of two or more triangles at a time: 8 B per triangle of the
+    // collapse's plan (32 B), which is not written before the tree is done
+    SahTiny* tiny = c->plan.as<SahTiny>();
+    static_assert(sizeof(SahTiny) / 2 <= 32, "the plan holds the queue");
+    HY_CUDA_TRY(cudaMemsetAsync(ctr, 0, CTR_COUNT * 4, s));
     const bool root_small = n <= small_max;
     SahRange* root = root_small ? c->sah_small.as<SahRange>() : c->sah_ranges[0].as<SahRange>();
     k_sah_root_init<<<1, 32, 0, s>>>(root, n);
@@ -662,8 +775,10 @@ int sah_tree_impl(HyCtx* c, uint32_t n, uint32_t* ord, uint32_t* ord2, uint32_t*
     }
     if (nsmall > 0) {
         k_sah_small<<<cdiv_u(nsmall, kSmallWarps), 32 * kSmallWarps, 0, s>>>(
-            c->sah_small.as<SahRange>(), nsmall, n, c->centroid.as<float4>(), c->tribox.as<float>(), ord, ord2, bvh2,
-            parent, ctr);
+            c->sah_small.as<SahRange>(), nsmall, n, c->centroid.as<float4>(), c->tribox.as<float>(), ord, ord2, tiny,
+            bvh2, parent, ctr);
+        k_sah_tiny<<<std::min<uint32_t>(cdiv_u(n / 2, 128), 16 * (uint32_t)c->num_sms), 128, 0, s>>>(
+            tiny, n, c->centroid.as<float4>(), c->tribox.as<float>(), ord, bvh2, parent, ctr);
         HY_CUDA_TRY(cudaGetLastError());
     }
     uint32_t h_err = 0;
