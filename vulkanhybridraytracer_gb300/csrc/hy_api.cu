@@ -476,8 +476,8 @@ void hy_destroy(HyCtx* c) {
     DevBuf* bufs[] = {&c->verts, &c->vattr, &c->idx, &c->prims, &c->xf, &c->nrm, &c->prim_tri0, &c->tri_prim,
                       &c->mats, &c->lights, &c->env[0], &c->env[1], &c->world, &c->tribox, &c->centroid,
                       &c->keys[0], &c->keys[1], &c->vals[0], &c->vals[1], &c->bvh2, &c->parent, &c->flags,
-                      &c->bounds, &c->lvl_ref[0], &c->lvl_ref[1], &c->plan, &c->ni, &c->nt, &c->ni_scan,
-                      &c->nt_scan, &c->scan_tmp, &c->hist, &c->total, &c->nodes, &c->tris, &c->node_ref,
+                      &c->bounds, &c->lvl_ref[0], &c->lvl_ref[1], &c->plan, &c->ni, &c->ni_scan,
+                      &c->scan_tmp, &c->hist, &c->total, &c->nodes, &c->tris, &c->node_ref,
                       &c->node_plan, &c->dstats,
                       &c->raw_shadow, &c->hist_prev, &c->host_in[0], &c->host_in[1], &c->host_in[2],
                       &c->host_in[3], &c->host_in[4], &c->host_in[5], &c->host_out_f, &c->host_out_8,

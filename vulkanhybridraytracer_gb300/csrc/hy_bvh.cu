@@ -10,9 +10,9 @@
 //   k_karras        Karras 2012 binary radix tree over (morton << 32 | id)
 //                   (HY_BUILD_LBVH), or the binned-SAH tree of hy_sah.cu
 //                   over the same order (HY_BUILD_SAH, the default)
-//   k_refit         bottom-up boxes, last-arriver-computes (no waiting)
-//   k_collapse_dp   slot budgets of the collapse by the surface area heuristic
-//                   (bottom up, last arriver computes)
+//   k_boxes_dp      bottom-up boxes and the slot budgets of the collapse by the surface
+//                   area heuristic, last arriver computes (no waiting); k_refit: the
+//                   boxes alone
 //   k_collapse_*    BFS collapse into compressed 8-wide nodes, one level per
 //                   launch pair with prefix sums for deterministic numbering
 //
@@ -209,6 +209,85 @@ int scan_exclusive(HyCtx* c, const uint32_t* in, uint32_t* out, uint32_t n, uint
     return HY_OK;
 }
 
+// The collapse's two counts per node as one 64-bit scan (both sums stay below 2^32),
+// in one launch where one block is enough.
+__device__ __forceinline__ unsigned long long block_excl_scan64(unsigned long long v, unsigned long long* sm,
+                                                                unsigned long long& total) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    unsigned long long x = v;
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) sm[w] = x;
+    __syncthreads();
+    if (w == 0) {
+        unsigned long long s = lane < (SCAN_T / 32) ? sm[lane] : 0ull;
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long y = __shfl_up_sync(0xffffffffu, s, o);
+            if (lane >= o) s += y;
+        }
+        if (lane < (SCAN_T / 32)) sm[lane] = s;
+    }
+    __syncthreads();
+    total = sm[SCAN_T / 32 - 1];
+    const unsigned long long base = w > 0 ? sm[w - 1] : 0ull;
+    __syncthreads();
+    return base + x - v;
+}
+__global__ void k_scan64_sums(const unsigned long long* __restrict__ in, uint32_t n,
+                              unsigned long long* __restrict__ sums) {
+    __shared__ unsigned long long sm[32];
+    const uint32_t base = blockIdx.x * SCAN_TILE + threadIdx.x * SCAN_I;
+    unsigned long long s = 0, tot;
+    for (int i = 0; i < SCAN_I; i++) if (base + i < n) s += in[base + i];
+    block_excl_scan64(s, sm, tot);
+    if (threadIdx.x == 0) sums[blockIdx.x] = tot;
+}
+__global__ void k_scan64_top(unsigned long long* sums, uint32_t nb, unsigned long long* total) {
+    __shared__ unsigned long long sm[32];
+    unsigned long long carry = 0;
+    for (uint32_t off = 0; off < nb; off += SCAN_T) {
+        const uint32_t i = off + threadIdx.x;
+        unsigned long long v = i < nb ? sums[i] : 0ull, tot;
+        const unsigned long long e = block_excl_scan64(v, sm, tot);
+        if (i < nb) sums[i] = carry + e;
+        carry += tot;
+    }
+    if (threadIdx.x == 0) *total = carry;
+}
+// sums null: a single block, which also gives the total
+__global__ void k_scan64_apply(const unsigned long long* __restrict__ in, uint32_t n,
+                               const unsigned long long* __restrict__ sums, unsigned long long* __restrict__ out,
+                               unsigned long long* total) {
+    __shared__ unsigned long long sm[32];
+    const uint32_t base = blockIdx.x * SCAN_TILE + threadIdx.x * SCAN_I;
+    unsigned long long v[SCAN_I], s = 0, tot;
+    for (int i = 0; i < SCAN_I; i++) { v[i] = base + i < n ? in[base + i] : 0ull; s += v[i]; }
+    unsigned long long run = block_excl_scan64(s, sm, tot) + (sums ? sums[blockIdx.x] : 0ull);
+    for (int i = 0; i < SCAN_I; i++) {
+        if (base + i < n) out[base + i] = run;
+        run += v[i];
+    }
+    if (!sums && threadIdx.x == 0) *total = tot;
+}
+
+static int scan_exclusive64(HyCtx* c, const unsigned long long* in, unsigned long long* out, uint32_t n,
+                            unsigned long long* d_total) {
+    const uint32_t nb = std::max<uint32_t>((n + SCAN_TILE - 1) / SCAN_TILE, 1);
+    unsigned long long* sums = nullptr;
+    if (nb > 1) {
+        int rc = ctx_alloc(c, c->scan_tmp, (size_t)nb * 8);
+        if (rc) return rc;
+        sums = c->scan_tmp.as<unsigned long long>();
+        k_scan64_sums<<<nb, SCAN_T, 0, c->stream>>>(in, n, sums);
+        k_scan64_top<<<1, SCAN_T, 0, c->stream>>>(sums, nb, d_total);
+    }
+    k_scan64_apply<<<nb, SCAN_T, 0, c->stream>>>(in, n, sums, out, d_total);
+    HY_CUDA_TRY(cudaGetLastError());
+    return HY_OK;
+}
+
 // ---------------------------------------------------------------------------------
 // stable LSD radix sort, 8-bit digits
 // ---------------------------------------------------------------------------------
@@ -392,15 +471,24 @@ __device__ __forceinline__ float surface(const Ref& b) {
 // order) are the oracle's.
 constexpr float kCostNode = 1.0f, kCostTri = 0.5f;
 
-__device__ __forceinline__ float dp_cost(uint32_t m, int i, const float* dpf, const uint32_t* order,
-                                         const float* tribox) {
-    if (m & kLeaf) return __fmul_rn(surface(load_ref(m, nullptr, order, tribox)), kCostTri);
-    return __ldcg(dpf + (size_t)m * 8 + i - 1);
+// The boxes of the binary tree (as k_refit) and the slot budgets in one climb.
+__device__ __forceinline__ void dp_child(uint32_t m, const float lo[3], const float hi[3], const float* dpf, float f[8]) {
+    if (m & kLeaf) {
+        Ref b;
+        for (int a = 0; a < 3; a++) { b.lo[a] = lo[a]; b.hi[a] = hi[a]; }
+        const float v = __fmul_rn(surface(b), kCostTri);
+#pragma unroll
+        for (int i = 0; i < 8; i++) f[i] = v;
+    } else {
+        const float4 p = __ldcg((const float4*)(dpf + (size_t)m * 8)), q = __ldcg((const float4*)(dpf + (size_t)m * 8) + 1);
+        f[0] = p.x; f[1] = p.y; f[2] = p.z; f[3] = p.w;
+        f[4] = q.x; f[5] = q.y; f[6] = q.z; f[7] = q.w;
+    }
 }
 
-__global__ void k_collapse_dp(const uint32_t* __restrict__ order, const float* __restrict__ tribox, uint32_t n,
-                              const uint32_t* __restrict__ bvh2, const uint32_t* __restrict__ parent,
-                              uint32_t* flags, float* dpf, uint8_t* dpk) {
+__global__ void k_boxes_dp(const uint32_t* __restrict__ order, const float* __restrict__ tribox, uint32_t n,
+                           uint32_t* bvh2, const uint32_t* __restrict__ parent, uint32_t* flags, float* dpf,
+                           uint8_t* dpk) {
     uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
     uint32_t p = parent[n - 1 + j];
@@ -408,21 +496,26 @@ __global__ void k_collapse_dp(const uint32_t* __restrict__ order, const float* _
         __threadfence();
         if (atomicAdd(flags + p, 1u) == 0u) return;  // the sibling's thread computes this node
         __threadfence();
-        const uint32_t* nd = bvh2 + (size_t)p * 10;
-        const uint32_t L = __ldcg(nd + 0), R = __ldcg(nd + 1);
-        float fl[8], fr[8];
-#pragma unroll
-        for (int i = 1; i <= 8; i++) {
-            fl[i - 1] = dp_cost(L, i, dpf, order, tribox);
-            fr[i - 1] = dp_cost(R, i, dpf, order, tribox);
-        }
+        uint32_t* nd = bvh2 + (size_t)p * 10;
+        const uint32_t L = __ldcg(nd + 0), R = __ldcg(nd + 1), first = __ldcg(nd + 2), last = __ldcg(nd + 3);
+        const uint32_t up = parent[p];
         Ref nb;
-        for (int a = 0; a < 3; a++) {
-            nb.lo[a] = __uint_as_float(__ldcg(nd + 4 + a));
-            nb.hi[a] = __uint_as_float(__ldcg(nd + 7 + a));
+        float fl[8], fr[8];
+        {
+            float l0[3], h0[3], l1[3], h1[3];
+            child_box(L, bvh2, order, tribox, l0, h0);
+            child_box(R, bvh2, order, tribox, l1, h1);
+            dp_child(L, l0, h0, dpf, fl);
+            dp_child(R, l1, h1, dpf, fr);
+            for (int a = 0; a < 3; a++) {
+                nb.lo[a] = fminf(l0[a], l1[a]);
+                nb.hi[a] = fmaxf(h0[a], h1[a]);
+                __stcg(nd + 4 + a, __float_as_uint(nb.lo[a]));
+                __stcg(nd + 7 + a, __float_as_uint(nb.hi[a]));
+            }
         }
         const float A = surface(nb);
-        const uint32_t cnt = __ldcg(nd + 3) - __ldcg(nd + 2) + 1;
+        const uint32_t cnt = last - first + 1;
         float best8 = INFINITY;
         int bk = 1;
 #pragma unroll
@@ -439,6 +532,7 @@ __global__ void k_collapse_dp(const uint32_t* __restrict__ order, const float* _
         for (int i = 2; i <= 8; i++) {
             float v = f[i - 2];
             int kk = 0;
+#pragma unroll
             for (int k = 1; k < i; k++) {
                 const float w = __fadd_rn(fl[k - 1], fr[i - k - 1]);
                 if (w < v) { v = w; kk = k; }
@@ -446,85 +540,115 @@ __global__ void k_collapse_dp(const uint32_t* __restrict__ order, const float* _
             f[i - 1] = v;
             kd[i] = (uint8_t)kk;
         }
-        float* fo = dpf + (size_t)p * 8;
-#pragma unroll
-        for (int i = 0; i < 8; i++) __stcg(fo + i, f[i]);
-        p = parent[p];
+        float4* fo = (float4*)(dpf + (size_t)p * 8);
+        __stcg(fo, make_float4(f[0], f[1], f[2], f[3]));
+        __stcg(fo + 1, make_float4(f[4], f[5], f[6], f[7]));
+        p = up;
     }
 }
 
-// plan: 8 BVH2 refs per node in slot order (0xffffffff = empty)
-__global__ void k_collapse_plan(const uint32_t* __restrict__ lvl, uint32_t m, const uint32_t* __restrict__ bvh2,
-                                const uint32_t* __restrict__ order, const float* __restrict__ tribox,
-                                const uint8_t* __restrict__ dpk, uint32_t* __restrict__ plan,
-                                uint32_t* __restrict__ ni, uint32_t* __restrict__ nt) {
-    uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= m) return;
-    uint32_t r = lvl[k];
-    // children: the node's 8 slots spread over its subtree by the slot budgets,
-    // left subtree first
-    uint32_t C[8];
+// plan: 8 BVH2 refs per node in slot order (0xffffffff = empty).  Eight lanes per
+// node: the first spreads the node's 8 slots over its subtree by the slot budgets,
+// then lane i holds child i and its cost in each slot, and each of the assignment's
+// steps takes the best (cost, then lowest child, then lowest slot) over the lanes.
+// counts[k]: (child nodes << 32) | leaf triangles.  (A thread per node with its 8 x 8
+// costs in local memory: 651 us for the 171k nodes of 1.5M triangles.)
+__global__ void __launch_bounds__(128) k_collapse_plan(const uint32_t* __restrict__ lvl, uint32_t m,
+                                                       const uint32_t* __restrict__ bvh2,
+                                                       const uint32_t* __restrict__ order,
+                                                       const float* __restrict__ tribox,
+                                                       const uint8_t* __restrict__ dpk, uint32_t* __restrict__ plan,
+                                                       unsigned long long* __restrict__ counts) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, k = t >> 3, li = t & 7u;
+    const uint32_t lane = threadIdx.x & 31, g0 = lane & ~7u;  // the group's first lane
+    const bool valid = k < m;
+    const uint32_t r = valid ? lvl[k] : kLeaf;
+    uint32_t mine = 0xffffffffu;  // this lane's child
     int nc = 0;
-    if (r & kLeaf) {
-        C[nc++] = r;
-    } else {
-        uint32_t sm_[8];
-        int si_[8], sp = 0;
-        const int k0 = dpk[(size_t)r * 9];
-        sm_[sp] = bvh2[(size_t)r * 10 + 1]; si_[sp++] = 8 - k0;
-        sm_[sp] = bvh2[(size_t)r * 10 + 0]; si_[sp++] = k0;
-        while (sp > 0) {
-            const uint32_t mm = sm_[--sp];
-            int i = si_[sp];
-            while (!(mm & kLeaf) && i > 1 && dpk[(size_t)mm * 9 + i] == 0) i--;
-            if ((mm & kLeaf) || i == 1) { C[nc++] = mm; continue; }
-            const int kk = dpk[(size_t)mm * 9 + i];
-            sm_[sp] = bvh2[(size_t)mm * 10 + 1]; si_[sp++] = i - kk;
-            sm_[sp] = bvh2[(size_t)mm * 10 + 0]; si_[sp++] = kk;
-        }
-    }
-    Ref nb = load_ref(r, bvh2, order, tribox);
-    float pc[3];
-    for (int a = 0; a < 3; a++) pc[a] = __fmul_rn(__fadd_rn(nb.lo[a], nb.hi[a]), 0.5f);
-    float cost[8][8];
-    uint32_t cnt[8];
-    for (int i = 0; i < nc; i++) {
-        Ref cb = load_ref(C[i], bvh2, order, tribox);
-        cnt[i] = cb.count;
-        float dd[3];
-        for (int a = 0; a < 3; a++) dd[a] = __fsub_rn(__fmul_rn(__fadd_rn(cb.lo[a], cb.hi[a]), 0.5f), pc[a]);
-        for (int sl = 0; sl < 8; sl++) {
-            float c0 = (sl & 1) ? dd[0] : -dd[0];
-            float c1 = (sl & 2) ? dd[1] : -dd[1];
-            float c2 = (sl & 4) ? dd[2] : -dd[2];
-            cost[i][sl] = __fadd_rn(__fadd_rn(c0, c1), c2);
-        }
-    }
-    int slot_of[8], child_in_slot[8];
-    for (int i = 0; i < 8; i++) { slot_of[i] = -1; child_in_slot[i] = -1; }
-    for (int it = 0; it < nc; it++) {
-        int bi = -1, bs = -1;
-        float bc = 0.f;
-        for (int i = 0; i < nc; i++) {
-            if (slot_of[i] >= 0) continue;
-            for (int sl = 0; sl < 8; sl++) {
-                if (child_in_slot[sl] >= 0) continue;
-                if (bi < 0 || cost[i][sl] > bc) { bi = i; bs = sl; bc = cost[i][sl]; }
+    {
+        // children, left subtree first; lane g0 walks, the others take theirs
+        uint32_t C[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) C[i] = 0xffffffffu;
+        if (valid && li == 0) {
+            if (r & kLeaf) {
+                C[nc++] = r;
+            } else {
+                uint32_t sm_[8];
+                int si_[8], sp = 0;
+                const int k0 = dpk[(size_t)r * 9];
+                sm_[sp] = bvh2[(size_t)r * 10 + 1]; si_[sp++] = 8 - k0;
+                sm_[sp] = bvh2[(size_t)r * 10 + 0]; si_[sp++] = k0;
+                while (sp > 0) {
+                    const uint32_t mm = sm_[--sp];
+                    int i = si_[sp];
+                    while (!(mm & kLeaf) && i > 1 && dpk[(size_t)mm * 9 + i] == 0) i--;
+                    if ((mm & kLeaf) || i == 1) { C[nc++] = mm; continue; }
+                    const int kk = dpk[(size_t)mm * 9 + i];
+                    sm_[sp] = bvh2[(size_t)mm * 10 + 1]; si_[sp++] = i - kk;
+                    sm_[sp] = bvh2[(size_t)mm * 10 + 0]; si_[sp++] = kk;
+                }
             }
         }
-        slot_of[bi] = bs;
-        child_in_slot[bs] = bi;
+        nc = __shfl_sync(0xffffffffu, nc, g0);
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const uint32_t c = __shfl_sync(0xffffffffu, C[i], g0);
+            if ((int)li == i) mine = c;
+        }
     }
-    uint32_t n_int = 0, n_tri = 0;
-    for (int sl = 0; sl < 8; sl++) {
-        int i = child_in_slot[sl];
-        plan[(size_t)k * 8 + sl] = i < 0 ? 0xffffffffu : C[i];
-        if (i < 0) continue;
-        if (cnt[i] > (uint32_t)kLeafMax) n_int++;
-        else n_tri += cnt[i];
+    const bool has = valid && (int)li < nc;
+    float dd[3] = {0.f, 0.f, 0.f};
+    uint32_t cnt = 0;
+    if (has) {
+        const Ref nb = load_ref(r, bvh2, order, tribox), cb = load_ref(mine, bvh2, order, tribox);
+        cnt = cb.count;
+        for (int a = 0; a < 3; a++)
+            dd[a] = __fsub_rn(__fmul_rn(__fadd_rn(cb.lo[a], cb.hi[a]), 0.5f),
+                              __fmul_rn(__fadd_rn(nb.lo[a], nb.hi[a]), 0.5f));
     }
-    ni[k] = n_int;
-    nt[k] = n_tri;
+    float cost[8];
+#pragma unroll
+    for (int sl = 0; sl < 8; sl++)
+        cost[sl] = __fadd_rn(__fadd_rn((sl & 1) ? dd[0] : -dd[0], (sl & 2) ? dd[1] : -dd[1]), (sl & 4) ? dd[2] : -dd[2]);
+    uint32_t taken = 0;  // slots
+    int slot = -1;       // this lane's
+    const int steps = __reduce_max_sync(0xffffffffu, nc);
+    for (int it = 0; it < steps; it++) {
+        // this child's best free slot, first of equals
+        int bs = -1;
+        float bc = 0.f;
+        if (has && slot < 0) {
+#pragma unroll
+            for (int sl = 0; sl < 8; sl++)
+                if (!((taken >> sl) & 1u) && (bs < 0 || cost[sl] > bc)) { bs = sl; bc = cost[sl]; }
+        }
+        // the group's best child, in order: only a strictly greater cost wins
+        int who = -1, ws = -1;
+        float wc = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int os = __shfl_sync(0xffffffffu, bs, g0 + i);
+            const float oc = __shfl_sync(0xffffffffu, bc, g0 + i);
+            if (os >= 0 && (who < 0 || oc > wc)) { who = i; ws = os; wc = oc; }
+        }
+        if (who >= 0) {
+            taken |= 1u << ws;
+            if (who == (int)li) slot = ws;
+        }
+    }
+    uint32_t at = 0xffffffffu;  // the child in slot li
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const int os = __shfl_sync(0xffffffffu, slot, g0 + i);
+        const uint32_t oc = __shfl_sync(0xffffffffu, mine, g0 + i);
+        if (os == (int)li) at = oc;
+    }
+    if (valid) plan[(size_t)k * 8 + li] = at;
+    unsigned long long v = !has ? 0ull : cnt > (uint32_t)kLeafMax ? 1ull << 32 : (unsigned long long)cnt;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (valid && li == 0) counts[k] = v;
 }
 
 // Node origin p = the node box's lo corner, per-axis power-of-two scale 2^e
@@ -563,7 +687,7 @@ __device__ __forceinline__ void quantize_node(const Ref& nb, const uint32_t* slo
 __global__ void k_collapse_emit(uint32_t m, uint32_t level_start, uint32_t tri_start, uint32_t node_off,
                                 uint32_t rec_off,
                                 const uint32_t* __restrict__ lvl, const uint32_t* __restrict__ plan,
-                                const uint32_t* __restrict__ ni_scan, const uint32_t* __restrict__ nt_scan,
+                                const unsigned long long* __restrict__ scan,
                                 const uint32_t* __restrict__ bvh2, const uint32_t* __restrict__ order,
                                 const float* __restrict__ tribox, const float4* __restrict__ world,
                                 Node8* __restrict__ nodes, float4* __restrict__ tris, uint32_t* __restrict__ next,
@@ -571,8 +695,9 @@ __global__ void k_collapse_emit(uint32_t m, uint32_t level_start, uint32_t tri_s
     uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= m) return;
     Ref nb = load_ref(lvl[k], bvh2, order, tribox);
-    uint32_t child_base = node_off + level_start + m + ni_scan[k];
-    uint32_t tri_base = rec_off + tri_start + nt_scan[k];
+    const uint32_t nodes_before = (uint32_t)(scan[k] >> 32), tris_before = (uint32_t)scan[k];
+    uint32_t child_base = node_off + level_start + m + nodes_before;
+    uint32_t tri_base = rec_off + tri_start + tris_before;
     const uint32_t* slots = plan + (size_t)k * 8;
     // kept for refits: the node's BVH2 subtree and its children in slot order
     node_ref[level_start + k] = lvl[k];
@@ -589,7 +714,7 @@ __global__ void k_collapse_emit(uint32_t m, uint32_t level_start, uint32_t tri_s
         if (cb.count > (uint32_t)kLeafMax) {
             imask |= 1u << sl;
             meta[wsel] |= 0x80u << sh;
-            next[ni_scan[k] + rank] = c;
+            next[nodes_before + rank] = c;
             rank++;
         } else {
             meta[wsel] |= ((cb.count << 5) | toff) << sh;
@@ -681,9 +806,8 @@ static int build_core(HyCtx* c, uint32_t n, uint32_t node_off, uint32_t rec_off,
         (rc = ctx_alloc(c, c->parent, (size_t)(2 * n) * 4)) ||
         (rc = ctx_alloc(c, c->flags, (size_t)std::max<uint32_t>(n, 1) * 4)) ||
         (rc = ctx_alloc(c, c->lvl_ref[0], (size_t)n * 4)) || (rc = ctx_alloc(c, c->lvl_ref[1], (size_t)n * 4)) ||
-        (rc = ctx_alloc(c, c->plan, (size_t)n * 32)) || (rc = ctx_alloc(c, c->ni, (size_t)n * 4)) ||
-        (rc = ctx_alloc(c, c->nt, (size_t)n * 4)) || (rc = ctx_alloc(c, c->ni_scan, (size_t)n * 4)) ||
-        (rc = ctx_alloc(c, c->nt_scan, (size_t)n * 4)) ||
+        (rc = ctx_alloc(c, c->plan, (size_t)n * 32)) || (rc = ctx_alloc(c, c->ni, (size_t)n * 8)) ||
+        (rc = ctx_alloc(c, c->ni_scan, (size_t)n * 8)) ||
         (rc = ctx_alloc(c, c->node_ref, (size_t)std::max<uint32_t>(n, 1) * 4)) ||
         (rc = ctx_alloc(c, c->node_plan, (size_t)std::max<uint32_t>(n, 1) * 32)) ||
         (rc = ctx_alloc(c, c->dp_cost, (size_t)std::max<uint32_t>(n, 1) * 32)) ||
@@ -727,38 +851,34 @@ static int build_core(HyCtx* c, uint32_t n, uint32_t node_off, uint32_t rec_off,
             k_karras<<<cdiv(n - 1, 256), 256, 0, s>>>(mort, ord, n, bvh2, c->parent.as<uint32_t>());
         }
         HY_CUDA_TRY(cudaMemsetAsync(c->flags.p, 0, (size_t)n * 4, s));
-        k_refit<<<cdiv(n, 256), 256, 0, s>>>(ord, c->tribox.as<float>(), n, bvh2, c->parent.as<uint32_t>(),
-                                             c->flags.as<uint32_t>());
-        HY_CUDA_TRY(cudaMemsetAsync(c->flags.p, 0, (size_t)n * 4, s));
-        k_collapse_dp<<<cdiv(n, 256), 256, 0, s>>>(ord, c->tribox.as<float>(), n, bvh2, c->parent.as<uint32_t>(),
-                                                   c->flags.as<uint32_t>(), c->dp_cost.as<float>(),
-                                                   c->dp_k.as<uint8_t>());
+        k_boxes_dp<<<cdiv(n, 256), 256, 0, s>>>(ord, c->tribox.as<float>(), n, bvh2, c->parent.as<uint32_t>(),
+                                                c->flags.as<uint32_t>(), c->dp_cost.as<float>(),
+                                                c->dp_k.as<uint8_t>());
     }
     HY_CUDA_TRY(cudaGetLastError());
     uint32_t level_start = 0, tri_start = 0, m = 1, depth = 0;
     int lv = 0;
-    uint32_t* tot = c->total.as<uint32_t>();
+    unsigned long long* tot = c->total.as<unsigned long long>();
+    unsigned long long* counts = c->ni.as<unsigned long long>();
+    unsigned long long* scan = c->ni_scan.as<unsigned long long>();
     while (m > 0) {
         const uint32_t* lvl = c->lvl_ref[lv].as<uint32_t>();
-        k_collapse_plan<<<cdiv(m, 128), 128, 0, s>>>(lvl, m, bvh2, ord, c->tribox.as<float>(),
-                                                     c->dp_k.as<uint8_t>(), c->plan.as<uint32_t>(),
-                                                     c->ni.as<uint32_t>(), c->nt.as<uint32_t>());
-        if ((rc = scan_exclusive(c, c->ni.as<uint32_t>(), c->ni_scan.as<uint32_t>(), m, tot))) return rc;
-        if ((rc = scan_exclusive(c, c->nt.as<uint32_t>(), c->nt_scan.as<uint32_t>(), m, tot + 1))) return rc;
+        k_collapse_plan<<<cdiv(m, 16), 128, 0, s>>>(lvl, m, bvh2, ord, c->tribox.as<float>(), c->dp_k.as<uint8_t>(),
+                                                    c->plan.as<uint32_t>(), counts);
+        if ((rc = scan_exclusive64(c, counts, scan, m, tot))) return rc;
         k_collapse_emit<<<cdiv(m, 128), 128, 0, s>>>(m, level_start, tri_start, node_off, rec_off, lvl,
-                                                     c->plan.as<uint32_t>(),
-                                                     c->ni_scan.as<uint32_t>(), c->nt_scan.as<uint32_t>(), bvh2, ord,
+                                                     c->plan.as<uint32_t>(), scan, bvh2, ord,
                                                      c->tribox.as<float>(), c->world.as<float4>(),
                                                      c->nodes.as<Node8>(), c->tris.as<float4>(),
                                                      c->lvl_ref[lv ^ 1].as<uint32_t>(), c->node_ref.as<uint32_t>(),
                                                      c->node_plan.as<uint32_t>());
         HY_CUDA_TRY(cudaGetLastError());
-        uint32_t h_tot[2];
+        unsigned long long* h_tot = c->h_stats;  // pinned
         HY_CUDA_TRY(cudaMemcpyAsync(h_tot, tot, 8, cudaMemcpyDeviceToHost, s));
         HY_CUDA_TRY(cudaStreamSynchronize(s));
         level_start += m;
-        tri_start += h_tot[1];
-        m = h_tot[0];
+        tri_start += (uint32_t)*h_tot;
+        m = (uint32_t)(*h_tot >> 32);
         lv ^= 1;
         depth++;
         if (depth > 256) return HY_ERR_TIMEOUT;

@@ -57,7 +57,7 @@ struct HyCtx {
     hy::DevBuf parent;      // n-1 internal + n leaves
     hy::DevBuf flags;       // refit arrival counters
     hy::DevBuf bounds;      // 6 orderable ints + build scratch
-    hy::DevBuf lvl_ref[2], plan, ni, nt, ni_scan, nt_scan;
+    hy::DevBuf lvl_ref[2], plan, ni, ni_scan;  // ni: (child nodes << 32) | leaf triangles per node, and its scan
     hy::DevBuf scan_tmp, hist, total;
     hy::DevBuf nodes, tris;
     hy::DevBuf node_ref, node_plan;  // per BVH8 node: its BVH2 subtree, its 8 slot children (refits)

@@ -25,12 +25,13 @@
 // level by four launches over chunks of kChunk triangles (bin: shared-memory
 // bins flushed with global atomics; eval: a block per range picks the split
 // and the chunks' output offsets; scatter: the stable partition into scratch
-// with a block scan; copy back).  Ranges of up to small_max triangles are
-// whole subtrees for one warp each (k_sah_small), which walks them with a
-// short explicit stack (the larger side pushed, the smaller taken first, so at
-// most log2(small_max) entries).  small_max (64..4096) is picked per build so
-// that about 16 warps per SM get a subtree; it changes the schedule only, not
-// the tree.
+// with a block scan; copy back).  Ranges of up to small_max triangles are split
+// by one warp each, a launch per level (k_sah_step, up to 8 launches); a warp walks what is
+// left of a subtree then (k_sah_small) with a short explicit stack (the larger side
+// pushed, the smaller taken first, so at most log2(small_max) entries).  Ranges of
+// up to 8 triangles are whole subtrees for one thread each (k_sah_tiny).
+// small_max (64..4096) is picked per build so that about 16 warps per SM start with
+// a range; it changes the schedule only, not the tree.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -64,7 +65,8 @@ static_assert(sizeof(SahRange) == 40, "SahRange layout");
 struct SahChunk { uint32_t node, start, end, first; };  // range slot, [start, end), the range's first chunk
 struct SahSplit { int axis, q; uint32_t m, child[2]; };  // child: 0 none, 1 << 30 | next-level slot, 2 << 30 | small slot
 
-enum { CTR_NEXT = 0, CTR_SMALL = 1, CTR_ROOT = 2, CTR_ERR = 3, CTR_TINY = 4, CTR_COUNT };
+enum { CTR_NEXT = 0, CTR_SMALL = 1, CTR_ROOT = 2, CTR_ERR = 3, CTR_TINY = 4, CTR_STEP = 5, CTR_COUNT = CTR_STEP + 8 };
+constexpr int kSteps = CTR_COUNT - CTR_STEP;  // launches of k_sah_step
 
 // ranges of up to kTiny triangles: whole subtrees for one thread each (k_sah_tiny)
 constexpr uint32_t kTiny = 8;
@@ -232,6 +234,16 @@ __global__ void k_sah_root_init(SahRange* r, uint32_t n) {
     }
 }
 
+// a root within small_max: queued for the warps (it sits at slot 0), or the threads
+__global__ void k_sah_root_queue(SahTiny* tiny, uint32_t n, uint32_t* ctr) {
+    if (n > kTiny) {
+        ctr[CTR_SMALL] = 1;
+    } else {
+        tiny[0] = SahTiny{0, n - 1, kNone, 0};
+        ctr[CTR_TINY] = 1;
+    }
+}
+
 __global__ void k_sah_root_bounds(const float4* __restrict__ cen, uint32_t n, SahRange* r) {
     int k[6];
     keys_init(k);
@@ -249,6 +261,10 @@ __global__ void k_sah_bins_init(int* __restrict__ gbins, uint32_t nwords) {
     }
 }
 
+// One chunk's triangles into shared bins, then into the range's.  A thread takes 8
+// consecutive triangles and adds runs of one bin at once: the order is spatially
+// coherent, so a warp's triangles share bins, and an atomic per triangle and word
+// queued 32 deep on one address (a level of 1.5M triangles: 93 us).
 __global__ void __launch_bounds__(256) k_sah_bin(const SahChunk* __restrict__ chunks,
                                                  const SahRange* __restrict__ ranges,
                                                  const uint32_t* __restrict__ ord, const float4* __restrict__ cen,
@@ -259,9 +275,41 @@ __global__ void __launch_bounds__(256) k_sah_bin(const SahChunk* __restrict__ ch
     const Axes x = axes_of(ranges[ch.node].ck);
     bins_clear(sb, threadIdx.x, blockDim.x);
     __syncthreads();
-    for (uint32_t i = ch.start + threadIdx.x; i < ch.end; i += blockDim.x) {
-        const uint32_t t = ord[i];
-        bin_one(sb, x, cen[t], box + (size_t)t * 6);
+    constexpr uint32_t kPer = kChunk / 256;
+    const uint32_t i0 = ch.start + threadIdx.x * kPer, i1 = min(i0 + kPer, ch.end);
+    int run_bin[3] = {-1, -1, -1}, run_n[3] = {0, 0, 0}, rl[3][3] = {}, rh[3][3] = {};
+    for (uint32_t i = i0; i <= i1 && i0 < i1; i++) {
+        int kl[3], kh[3], bin[3] = {-1, -1, -1};
+        if (i < i1) {
+            const uint32_t t = ord[i];
+            const float4 ce = cen[t];
+            const float* bx = box + (size_t)t * 6;
+#pragma unroll
+            for (int k = 0; k < 3; k++) { kl[k] = okey(bx[k]); kh[k] = okey(bx[3 + k]); }
+            const float cc[3] = {ce.x, ce.y, ce.z};
+#pragma unroll
+            for (int a = 0; a < 3; a++)
+                if (x.ok[a]) bin[a] = sah_bin(cc[a], x.lo[a], x.scale[a]);
+        }
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            if (bin[a] == run_bin[a] && i < i1) {
+                run_n[a]++;
+#pragma unroll
+                for (int k = 0; k < 3; k++) { rl[a][k] = min(rl[a][k], kl[k]); rh[a][k] = max(rh[a][k], kh[k]); }
+                continue;
+            }
+            if (run_bin[a] >= 0) {
+                int* e = sb + a * kAxisWords + run_bin[a] * kBinWords;
+                atomicAdd(e, run_n[a]);
+#pragma unroll
+                for (int k = 0; k < 3; k++) { atomicMin(e + 1 + k, rl[a][k]); atomicMax(e + 4 + k, rh[a][k]); }
+            }
+            run_bin[a] = bin[a];
+            run_n[a] = 1;
+#pragma unroll
+            for (int k = 0; k < 3; k++) { rl[a][k] = kl[k]; rh[a][k] = kh[k]; }
+        }
     }
     __syncthreads();
     int* gb = gbins + (size_t)ch.node * kNodeBinWords;
@@ -286,8 +334,8 @@ __global__ void __launch_bounds__(256) k_sah_eval(const SahRange* __restrict__ r
                                                   const uint32_t* __restrict__ first_chunk,
                                                   const uint32_t* __restrict__ ccnt, uint32_t* __restrict__ coff,
                                                   SahSplit* __restrict__ split, SahRange* __restrict__ next,
-                                                  SahRange* __restrict__ small, uint32_t n, uint32_t small_max,
-                                                  uint32_t* __restrict__ bvh2, uint32_t* __restrict__ parent,
+                                                  SahRange* __restrict__ small, SahTiny* __restrict__ tiny,
+                                                  uint32_t n, uint32_t small_max, uint32_t* __restrict__ bvh2, uint32_t* __restrict__ parent,
                                                   uint32_t* __restrict__ ctr) {
     __shared__ unsigned long long s_key[3];
     __shared__ uint32_t s_part[256];
@@ -336,6 +384,10 @@ __global__ void __launch_bounds__(256) k_sah_eval(const SahRange* __restrict__ r
             const uint32_t cs = cl[s] - cf[s] + 1;
             sp.child[s] = 0;
             if (cs < 2) continue;
+            if (cs <= kTiny) {
+                tiny[atomicAdd(ctr + CTR_TINY, 1u)] = SahTiny{cf[s], cl[s], id, (uint32_t)s};
+                continue;
+            }
             SahRange ch;
             ch.f = cf[s];
             ch.l = cl[s];
@@ -464,11 +516,124 @@ __global__ void k_sah_copy(const SahChunk* __restrict__ chunks, const uint32_t* 
     for (uint32_t i = ch.start + threadIdx.x; i < ch.end; i += blockDim.x) ord[i] = ord2[i];
 }
 
-// ---- one warp per range of up to small_max triangles --------------------------
+// ---- one warp per range of kTiny + 1 .. small_max triangles ---------------------
 constexpr int kSmallWarps = 4;
 
-__global__ void __launch_bounds__(32 * kSmallWarps) k_sah_small(const SahRange* __restrict__ tasks, uint32_t ntask,
-                                                                uint32_t n, const float4* __restrict__ cen,
+// One range split by a warp: its triangles reordered in place, its node written.
+// Returns the split position; kl, kr: the centroid bounds of the sides.
+__device__ __forceinline__ uint32_t split_range(const SahRange& cur, int* bins, uint32_t n,
+                                                const float4* __restrict__ cen, const float* __restrict__ box,
+                                                uint32_t* ord, uint32_t* ord2, uint32_t* bvh2, uint32_t* parent,
+                                                uint32_t* ctr, int kl[6], int kr[6]) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t f = cur.f, l = cur.l, c = l - f + 1;
+    const Axes x = axes_of(cur.ck);
+    unsigned long long best = ~0ull;
+    if (x.ok[0] || x.ok[1] || x.ok[2]) {
+        bins_clear(bins, lane, 32);
+        __syncwarp();
+        for (uint32_t i = f + lane; i <= l; i += 32) {
+            const uint32_t t = ord[i];
+            bin_one(bins, x, cen[t], box + (size_t)t * 6);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            if (!x.ok[a]) continue;
+            const unsigned long long k = sweep_axis(bins + a * kAxisWords, a, lane);
+            best = k < best ? k : best;
+        }
+        best = warp_min_u64(best);
+    }
+    keys_init(kl);
+    keys_init(kr);
+    uint32_t m;
+    if (best != ~0ull) {
+        const int ba = (int)((uint32_t)best / kBins), bq = (int)((uint32_t)best % kBins);
+        const uint32_t cnt = lane <= (uint32_t)bq ? (uint32_t)bins[ba * kAxisWords + lane * kBinWords] : 0u;
+        m = f + __reduce_add_sync(kFull, cnt);
+        uint32_t nl = 0, nr = 0;
+        const uint32_t lt = (1u << lane) - 1u;
+        for (uint32_t i0 = f; i0 <= l; i0 += 32) {
+            const uint32_t i = i0 + lane;
+            const bool valid = i <= l;
+            uint32_t t = 0;
+            float4 ce = make_float4(0.f, 0.f, 0.f, 0.f);
+            bool left = false;
+            if (valid) {
+                t = ord[i];
+                ce = cen[t];
+                const float cc = ba == 0 ? ce.x : (ba == 1 ? ce.y : ce.z);
+                left = sah_bin(cc, x.lo[ba], x.scale[ba]) <= bq;
+            }
+            const uint32_t L = __ballot_sync(kFull, left), V = __ballot_sync(kFull, valid);
+            if (valid) {
+                ord2[left ? f + nl + __popc(L & lt) : m + nr + __popc(~L & V & lt)] = t;
+                if (left) keys_add(kl, ce);
+                else keys_add(kr, ce);
+            }
+            nl += __popc(L);
+            nr += __popc(~L & V);
+        }
+        __syncwarp();
+        for (uint32_t i = f + lane; i <= l; i += 32) ord[i] = ord2[i];
+        __syncwarp();
+    } else {
+        m = f + c / 2;
+        for (uint32_t i = f + lane; i <= l; i += 32) {
+            const float4 ce = cen[ord[i]];
+            if (i < m) keys_add(kl, ce);
+            else keys_add(kr, ce);
+        }
+    }
+    keys_warp(kl);
+    keys_warp(kr);
+    if (lane == 0) write_node(m - 1, f, l, m, cur.parent, cur.side, n, bvh2, parent, ctr);
+    return m;
+}
+
+__device__ __forceinline__ SahRange side_range(uint32_t f, uint32_t l, uint32_t node, uint32_t side, const int k[6]) {
+    SahRange r;
+    r.f = f; r.l = l; r.parent = node; r.side = side;
+#pragma unroll
+    for (int j = 0; j < 6; j++) r.ck[j] = k[j];
+    return r;
+}
+
+// One split per queued range: the sides go to the next queue (or the tiny one), so the
+// warps of a launch grow from level to level instead of walking one subtree each (a
+// chain of 100 to 200 splits of 7 us on 16 warps per SM).
+__global__ void __launch_bounds__(32 * kSmallWarps) k_sah_step(const SahRange* __restrict__ in,
+                                                               const uint32_t* __restrict__ n_in,
+                                                               SahRange* __restrict__ out, uint32_t* __restrict__ n_out,
+                                                               uint32_t n, const float4* __restrict__ cen,
+                                                               const float* __restrict__ box, uint32_t* ord,
+                                                               uint32_t* ord2, SahTiny* __restrict__ tiny,
+                                                               uint32_t* __restrict__ bvh2,
+                                                               uint32_t* __restrict__ parent,
+                                                               uint32_t* __restrict__ ctr) {
+    __shared__ int s_bins[kSmallWarps][kNodeBinWords];
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, tasks = *n_in;
+    for (uint32_t task = blockIdx.x * kSmallWarps + w; task < tasks; task += gridDim.x * kSmallWarps) {
+        const SahRange cur = in[task];
+        int kl[6], kr[6];
+        const uint32_t m = split_range(cur, s_bins[w], n, cen, box, ord, ord2, bvh2, parent, ctr, kl, kr);
+        if (lane == 0) {
+            const uint32_t f[2] = {cur.f, m}, l[2] = {m - 1, cur.l};
+            for (uint32_t s = 0; s < 2; s++) {
+                const uint32_t c = l[s] - f[s] + 1;
+                if (c > kTiny) out[atomicAdd(n_out, 1u)] = side_range(f[s], l[s], m - 1, s, s ? kr : kl);
+                else if (c >= 2) tiny[atomicAdd(ctr + CTR_TINY, 1u)] = SahTiny{f[s], l[s], m - 1, s};
+            }
+        }
+        __syncwarp();
+    }
+}
+
+// What is left after the steps: a warp walks each range's whole subtree.
+__global__ void __launch_bounds__(32 * kSmallWarps) k_sah_small(const SahRange* __restrict__ in,
+                                                                const uint32_t* __restrict__ n_in, uint32_t n,
+                                                                const float4* __restrict__ cen,
                                                                 const float* __restrict__ box, uint32_t* ord,
                                                                 uint32_t* ord2, SahTiny* __restrict__ tiny,
                                                                 uint32_t* __restrict__ bvh2,
@@ -476,111 +641,40 @@ __global__ void __launch_bounds__(32 * kSmallWarps) k_sah_small(const SahRange* 
                                                                 uint32_t* __restrict__ ctr) {
     __shared__ int s_bins[kSmallWarps][kNodeBinWords];
     __shared__ SahRange s_stack[kSmallWarps][kStackMax];
-    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const uint32_t task = blockIdx.x * kSmallWarps + w;
-    if (task >= ntask) return;
-    int* bins = s_bins[w];
-    SahRange cur = tasks[task];
-    int sp = 0;
-    auto queue_tiny = [&](uint32_t f, uint32_t l, uint32_t par, uint32_t side) {
-        if (lane == 0) tiny[atomicAdd(ctr + CTR_TINY, 1u)] = SahTiny{f, l, par, side};
-    };
-    if (cur.l - cur.f + 1 <= kTiny) {
-        queue_tiny(cur.f, cur.l, cur.parent, cur.side);
-        return;
-    }
-    for (;;) {
-        const uint32_t f = cur.f, l = cur.l, c = l - f + 1;
-        const Axes x = axes_of(cur.ck);
-        unsigned long long best = ~0ull;
-        if (x.ok[0] || x.ok[1] || x.ok[2]) {
-            bins_clear(bins, lane, 32);
-            __syncwarp();
-            for (uint32_t i = f + lane; i <= l; i += 32) {
-                const uint32_t t = ord[i];
-                bin_one(bins, x, cen[t], box + (size_t)t * 6);
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, tasks = *n_in;
+    for (uint32_t task = blockIdx.x * kSmallWarps + w; task < tasks; task += gridDim.x * kSmallWarps) {
+        SahRange cur = in[task];
+        int sp = 0;
+        for (;;) {
+            int kl[6], kr[6];
+            const uint32_t f = cur.f, l = cur.l;
+            const uint32_t m = split_range(cur, s_bins[w], n, cen, box, ord, ord2, bvh2, parent, ctr, kl, kr);
+            const uint32_t nl = m - f, nr = l - m + 1;
+            if (lane == 0) {
+                if (nl >= 2 && nl <= kTiny) tiny[atomicAdd(ctr + CTR_TINY, 1u)] = SahTiny{f, m - 1, m - 1, 0};
+                if (nr >= 2 && nr <= kTiny) tiny[atomicAdd(ctr + CTR_TINY, 1u)] = SahTiny{m, l, m - 1, 1};
             }
-            __syncwarp();
-#pragma unroll
-            for (int a = 0; a < 3; a++) {
-                if (!x.ok[a]) continue;
-                const unsigned long long k = sweep_axis(bins + a * kAxisWords, a, lane);
-                best = k < best ? k : best;
-            }
-            best = warp_min_u64(best);
-        }
-        int kl[6], kr[6];
-        keys_init(kl);
-        keys_init(kr);
-        uint32_t m;
-        if (best != ~0ull) {
-            const int ba = (int)((uint32_t)best / kBins), bq = (int)((uint32_t)best % kBins);
-            const uint32_t cnt = lane <= (uint32_t)bq ? (uint32_t)bins[ba * kAxisWords + lane * kBinWords] : 0u;
-            m = f + __reduce_add_sync(kFull, cnt);
-            uint32_t nl = 0, nr = 0;
-            const uint32_t lt = (1u << lane) - 1u;
-            for (uint32_t i0 = f; i0 <= l; i0 += 32) {
-                const uint32_t i = i0 + lane;
-                const bool valid = i <= l;
-                uint32_t t = 0;
-                float4 ce = make_float4(0.f, 0.f, 0.f, 0.f);
-                bool left = false;
-                if (valid) {
-                    t = ord[i];
-                    ce = cen[t];
-                    const float cc = ba == 0 ? ce.x : (ba == 1 ? ce.y : ce.z);
-                    left = sah_bin(cc, x.lo[ba], x.scale[ba]) <= bq;
+            const SahRange L = side_range(f, m - 1, m - 1, 0, kl), R = side_range(m, l, m - 1, 1, kr);
+            const bool li = nl > kTiny, ri = nr > kTiny;
+            if (li && ri) {
+                const bool lsmall = nl <= nr;
+                if (sp >= kStackMax) {  // cannot happen (the stack holds at most log2(kSmallMaxCap) ranges)
+                    if (lane == 0) atomicExch(ctr + CTR_ERR, 1u);
+                    return;
                 }
-                const uint32_t L = __ballot_sync(kFull, left), V = __ballot_sync(kFull, valid);
-                if (valid) {
-                    ord2[left ? f + nl + __popc(L & lt) : m + nr + __popc(~L & V & lt)] = t;
-                    if (left) keys_add(kl, ce);
-                    else keys_add(kr, ce);
-                }
-                nl += __popc(L);
-                nr += __popc(~L & V);
+                if (lane == 0) s_stack[w][sp] = lsmall ? R : L;
+                sp++;
+                cur = lsmall ? L : R;
+            } else if (li) {
+                cur = L;
+            } else if (ri) {
+                cur = R;
+            } else {
+                if (sp == 0) break;
+                __syncwarp();
+                cur = s_stack[w][--sp];
             }
             __syncwarp();
-            for (uint32_t i = f + lane; i <= l; i += 32) ord[i] = ord2[i];
-            __syncwarp();
-        } else {
-            m = f + c / 2;
-            for (uint32_t i = f + lane; i <= l; i += 32) {
-                const float4 ce = cen[ord[i]];
-                if (i < m) keys_add(kl, ce);
-                else keys_add(kr, ce);
-            }
-        }
-        keys_warp(kl);
-        keys_warp(kr);
-        const uint32_t id = m - 1;
-        if (lane == 0) write_node(id, f, l, m, cur.parent, cur.side, n, bvh2, parent, ctr);
-        const uint32_t nleft = m - f, nright = l - m + 1;
-        if (nleft >= 2 && nleft <= kTiny) queue_tiny(f, m - 1, id, 0);
-        if (nright >= 2 && nright <= kTiny) queue_tiny(m, l, id, 1);
-        const bool li = nleft > kTiny, ri = nright > kTiny;
-        SahRange L, R;
-        L.f = f; L.l = m - 1; L.parent = id; L.side = 0;
-        R.f = m; R.l = l; R.parent = id; R.side = 1;
-#pragma unroll
-        for (int k = 0; k < 6; k++) { L.ck[k] = kl[k]; R.ck[k] = kr[k]; }
-        if (li && ri) {
-            const bool lsmall = (m - f) <= (l - m + 1);
-            if (sp >= kStackMax) {  // cannot happen (the stack holds at most log2(kSmallMaxCap) ranges)
-                if (lane == 0) atomicExch(ctr + CTR_ERR, 1u);
-                return;
-            }
-            if (lane == 0) s_stack[w][sp] = lsmall ? R : L;
-            sp++;
-            cur = lsmall ? L : R;
-        } else if (li) {
-            cur = L;
-        } else if (ri) {
-            cur = R;
-        } else {
-            if (sp == 0) break;
-            __syncwarp();
-            cur = s_stack[w][--sp];
         }
         __syncwarp();
     }
@@ -696,12 +790,12 @@ int sah_tree_impl(HyCtx* c, uint32_t n, uint32_t* ord, uint32_t* ord2, uint32_t*
     uint32_t small_max = 64;
     while (small_max < kSmallMaxCap && (uint64_t)small_max * 16u * (uint32_t)c->num_sms < n) small_max <<= 1;
     const uint32_t bigcap = n / (small_max + 1) + 2;
-    const uint32_t smallcap = n / 2 + 2;
+    const uint32_t smallcap = n / (kTiny + 1) + 2;  // ranges above kTiny triangles at a time
     const uint32_t chunkcap = n / kChunk + bigcap + 2;
     int rc;
     if ((rc = ctx_alloc(c, c->sah_ranges[0], (size_t)bigcap * sizeof(SahRange))) ||
         (rc = ctx_alloc(c, c->sah_ranges[1], (size_t)bigcap * sizeof(SahRange))) ||
-        (rc = ctx_alloc(c, c->sah_small, (size_t)smallcap * sizeof(SahRange))) ||
+        (rc = ctx_alloc(c, c->sah_small, (size_t)smallcap * 2 * sizeof(SahRange))) ||
         (rc = ctx_alloc(c, c->sah_bins, (size_t)bigcap * kNodeBinWords * 4)) ||
         (rc = ctx_alloc(c, c->sah_split, (size_t)bigcap * sizeof(SahSplit))) ||
         (rc = ctx_alloc(c, c->sah_chunks, (size_t)chunkcap * sizeof(SahChunk))) ||
@@ -721,11 +815,8 @@ int sah_tree_impl(HyCtx* c, uint32_t n, uint32_t* ord, uint32_t* ord2, uint32_t*
     k_sah_root_bounds<<<std::min<uint32_t>(cdiv_u(n, 256), 4 * (uint32_t)c->num_sms), 256, 0, s>>>(
         c->centroid.as<float4>(), n, root);
     HY_CUDA_TRY(cudaGetLastError());
-    uint32_t nbig = root_small ? 0 : 1, nsmall = root_small ? 1 : 0;
-    if (root_small) {
-        const uint32_t one = 1;
-        HY_CUDA_TRY(cudaMemcpyAsync(ctr + CTR_SMALL, &one, 4, cudaMemcpyHostToDevice, s));
-    }
+    uint32_t nbig = root_small ? 0 : 1;
+    if (root_small) k_sah_root_queue<<<1, 1, 0, s>>>(tiny, n, ctr);
     std::vector<SahRange> h_ranges;
     std::vector<SahChunk> h_chunks;
     std::vector<uint32_t> h_first;
@@ -759,7 +850,7 @@ int sah_tree_impl(HyCtx* c, uint32_t n, uint32_t* ord, uint32_t* ord2, uint32_t*
                                       c->sah_bins.as<int>(), c->sah_ccnt.as<uint32_t>());
         k_sah_eval<<<nbig, 256, 0, s>>>(ranges, c->sah_bins.as<int>(), c->sah_first.as<uint32_t>(),
                                         c->sah_ccnt.as<uint32_t>(), c->sah_coff.as<uint32_t>(),
-                                        c->sah_split.as<SahSplit>(), next, c->sah_small.as<SahRange>(), n,
+                                        c->sah_split.as<SahSplit>(), next, c->sah_small.as<SahRange>(), tiny, n,
                                         small_max, bvh2, parent, ctr);
         k_sah_scatter<<<nch, 256, 0, s>>>(chunks, ranges, c->sah_split.as<SahSplit>(), c->sah_coff.as<uint32_t>(),
                                           ord, ord2, c->centroid.as<float4>(), next, c->sah_small.as<SahRange>());
@@ -769,18 +860,30 @@ int sah_tree_impl(HyCtx* c, uint32_t n, uint32_t* ord, uint32_t* ord2, uint32_t*
         HY_CUDA_TRY(cudaMemcpyAsync(h_ctr, ctr, 8, cudaMemcpyDeviceToHost, s));
         HY_CUDA_TRY(cudaStreamSynchronize(s));
         nbig = h_ctr[CTR_NEXT];
-        nsmall = h_ctr[CTR_SMALL];
-        if (nbig > bigcap || nsmall > smallcap) return HY_ERR_CUDA;
+        if (nbig > bigcap || h_ctr[CTR_SMALL] > smallcap) return HY_ERR_CUDA;
         cur ^= 1;
     }
-    if (nsmall > 0) {
-        k_sah_small<<<cdiv_u(nsmall, kSmallWarps), 32 * kSmallWarps, 0, s>>>(
-            c->sah_small.as<SahRange>(), nsmall, n, c->centroid.as<float4>(), c->tribox.as<float>(), ord, ord2, tiny,
-            bvh2, parent, ctr);
-        k_sah_tiny<<<std::min<uint32_t>(cdiv_u(n / 2, 128), 16 * (uint32_t)c->num_sms), 128, 0, s>>>(
-            tiny, n, c->centroid.as<float4>(), c->tribox.as<float>(), ord, bvh2, parent, ctr);
-        HY_CUDA_TRY(cudaGetLastError());
+    // the small ranges: launches of one split per range, from one half of the queue
+    // buffer to the other, then the rest, then the tiny ones
+    if (n > kTiny) {
+        SahRange* q[2] = {c->sah_small.as<SahRange>(), c->sah_small.as<SahRange>() + smallcap};
+        const uint32_t blocks = std::min<uint32_t>(cdiv_u(smallcap, kSmallWarps), 8 * (uint32_t)c->num_sms);
+        const uint32_t* n_in = ctr + CTR_SMALL;
+        int at = 0, steps = 0;
+        while (steps < kSteps && (kTiny << steps) < small_max) steps++;
+        for (int k = 0; k < steps; k++) {
+            k_sah_step<<<blocks, 32 * kSmallWarps, 0, s>>>(q[at], n_in, q[at ^ 1], ctr + CTR_STEP + k, n,
+                                                           c->centroid.as<float4>(), c->tribox.as<float>(), ord, ord2,
+                                                           tiny, bvh2, parent, ctr);
+            n_in = ctr + CTR_STEP + k;
+            at ^= 1;
+        }
+        k_sah_small<<<blocks, 32 * kSmallWarps, 0, s>>>(q[at], n_in, n, c->centroid.as<float4>(), c->tribox.as<float>(),
+                                                        ord, ord2, tiny, bvh2, parent, ctr);
     }
+    k_sah_tiny<<<std::min<uint32_t>(cdiv_u(n / 2, 128), 16 * (uint32_t)c->num_sms), 128, 0, s>>>(
+        tiny, n, c->centroid.as<float4>(), c->tribox.as<float>(), ord, bvh2, parent, ctr);
+    HY_CUDA_TRY(cudaGetLastError());
     uint32_t h_err = 0;
     HY_CUDA_TRY(cudaMemcpyAsync(&h_err, ctr + CTR_ERR, 4, cudaMemcpyDeviceToHost, s));
     HY_CUDA_TRY(cudaMemcpyAsync(d_root, ctr + CTR_ROOT, 4, cudaMemcpyDeviceToDevice, s));
