@@ -425,76 +425,117 @@ __global__ void __launch_bounds__(128, MINB) k_pixels(const SceneDev S, const Pa
 }
 
 // postFragment.frag:9-20: rgb = pow(max(rgb, 0.001), 1/2.2) per pixel of the final
-// image (a full-screen quad sampling it NEAREST at texel centres), alpha kept
-__global__ void __launch_bounds__(256) k_post(const uint8_t* __restrict__ in8, const float4* __restrict__ inf,
-                                              uint32_t n, uchar4* __restrict__ out) {
+// image (a full-screen quad sampling it NEAREST at texel centres), alpha kept.  An
+// 8-bit image has 256 values: a block computes each once into a table and takes
+// kPostPixels pixels (three powf per pixel: 1700x900 17 us).
+constexpr uint32_t kPostPixels = 2048;
+__device__ __forceinline__ uint8_t post_channel(float v) { return quant8(powf(fmaxf(v, 0.001f), 1.0f / 2.2f)); }
+__global__ void __launch_bounds__(256) k_post8(const uint32_t* __restrict__ in, uint32_t n, uint32_t* __restrict__ out) {
+    __shared__ uint8_t s_tab[256];
+    s_tab[threadIdx.x] = post_channel(__fdiv_rn((float)threadIdx.x, 255.f));
+    __syncthreads();
+    const uint32_t end = min(n, (blockIdx.x + 1) * kPostPixels);
+    for (uint32_t i = blockIdx.x * kPostPixels + threadIdx.x; i < end; i += 256) {
+        const uint32_t q = in[i];  // B, G, R, A bytes; A / 255 back to 8 bits is A
+        out[i] = s_tab[q & 0xffu] | (uint32_t)s_tab[(q >> 8) & 0xffu] << 8 | (uint32_t)s_tab[(q >> 16) & 0xffu] << 16 |
+                 (q & 0xff000000u);
+    }
+}
+__global__ void __launch_bounds__(256) k_post(const float4* __restrict__ in, uint32_t n, uchar4* __restrict__ out) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    float4 c;
-    if (in8) {
-        const uchar4 q = reinterpret_cast<const uchar4*>(in8)[i];  // B, G, R, A bytes
-        c = make_float4(__fdiv_rn((float)q.z, 255.f), __fdiv_rn((float)q.y, 255.f), __fdiv_rn((float)q.x, 255.f),
-                        __fdiv_rn((float)q.w, 255.f));
-    } else {
-        c = inf[i];
-    }
-    const float gamma = 1.0f / 2.2f;
-    const float r = powf(fmaxf(c.x, 0.001f), gamma), g = powf(fmaxf(c.y, 0.001f), gamma),
-                b = powf(fmaxf(c.z, 0.001f), gamma);
-    out[i] = make_uchar4(quant8(b), quant8(g), quant8(r), quant8(c.w));
+    const float4 c = in[i];
+    out[i] = make_uchar4(post_channel(c.z), post_channel(c.y), post_channel(c.x), quant8(c.w));
 }
 
 cudaError_t launch_post(const uint8_t* in8, const float* inf, uint32_t n, uint8_t* out, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
-    k_post<<<(n + 255) / 256, 256, 0, s>>>(in8, reinterpret_cast<const float4*>(inf), n,
-                                            reinterpret_cast<uchar4*>(out));
+    if (in8)
+        k_post8<<<(n + kPostPixels - 1) / kPostPixels, 256, 0, s>>>(reinterpret_cast<const uint32_t*>(in8), n,
+                                                                    reinterpret_cast<uint32_t*>(out));
+    else
+        k_post<<<(n + 255) / 256, 256, 0, s>>>(reinterpret_cast<const float4*>(inf), n, reinterpret_cast<uchar4*>(out));
     return cudaGetLastError();
 }
 
-// blur.comp:35-81, reset-frame branch and running mean, one texel per thread
-__global__ void k_accumulate(const AccumParams A) {
-    uint32_t x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (x >= A.blur_w || y >= A.blur_h) return;
+// blur.comp:35-81, reset-frame branch and running mean, one texel per thread.  The
+// reset frame's 3x3 clamp reads a block's texels of one light from shared memory (each
+// from DRAM once instead of nine times through L1), and 8-bit images are compared as
+// bytes and turned into their n / 255 through a table: n / 255 grows with n, so the
+// clamp's bounds are the bytes' (1700x900 x 3 lights 76 us before).
+constexpr int kBlurW = 32, kBlurH = 16;
+template <bool U8>
+__global__ void __launch_bounds__(kBlurW * kBlurH) k_accumulate(const AccumParams A) {
+    using T = std::conditional_t<U8, uint8_t, float>;
+    __shared__ T s_tile[kBlurH + 2][kBlurW + 4];
+    __shared__ float s_unorm[U8 ? 256 : 1];
+    const uint32_t tid = threadIdx.x, lx = tid % kBlurW, ly = tid / kBlurW;
+    const uint32_t x = blockIdx.x * kBlurW + lx, y = blockIdx.y * kBlurH + ly;
+    const bool present = x < A.blur_w && y < A.blur_h;
     const size_t plane = (size_t)A.W * A.H, pix = (size_t)y * A.W + x;
-    float rx = 0.f;
-    if (A.frame <= 0) {
-        float4 mo = fetch_texel(A.motion, A.motion_fmt, pix);
-        rx = __fsub_rn(__fmul_rn(mo.x, 2.0f), 1.0f);
+    if (U8 && tid < 256) s_unorm[tid] = __fdiv_rn((float)tid, 255.0f);
+    auto value = [&](T v) -> float {
+        if constexpr (U8) return s_unorm[v];
+        else return v;
+    };
+    const T* raw = (const T*)A.shadow;
+    T* hist = (T*)A.hist;
+    auto store = [&](size_t i, float v) {
+        if constexpr (U8) hist[i] = quant8(v);
+        else hist[i] = v;
+    };
+    if (A.frame > 0) {
+        __syncthreads();
+        if (!present) return;
+        const float a = __fdiv_rn(1.0f, __fadd_rn((float)A.frame, 1.0f));
+        for (uint32_t l = 0; l < A.num_lights; l++) {
+            const size_t i = l * plane + pix;
+            store(i, __fadd_rn(__fmul_rn(value(hist[i]), __fsub_rn(1.0f, a)), __fmul_rn(value(raw[i]), a)));
+        }
+        return;
     }
+    // blur.comp:53: the y term reuses the x motion (vec2(float, vec2) constructor)
+    bool inside = false;
+    size_t from = 0;
+    if (present) {
+        const float4 mo = fetch_texel(A.motion, A.motion_fmt, pix);
+        const float rx = __fsub_rn(__fmul_rn(mo.x, 2.0f), 1.0f);
+        const float sx = __fadd_rn((float)x, __fmul_rn(rx, (float)A.W));
+        const float sy = __fadd_rn((float)y, __fmul_rn(rx, (float)A.H));
+        if (sx > -2147483648.f && sx < 2147483647.f && sy > -2147483648.f && sy < 2147483647.f) {
+            const int ix = (int)sx, iy = (int)sy;
+            inside = ix >= 0 && iy >= 0 && ix < (int)A.W && iy < (int)A.H;
+            if (inside) from = (size_t)iy * A.W + ix;
+        }
+    }
+    const T* prev = (const T*)A.hist_prev;
     for (uint32_t l = 0; l < A.num_lights; l++) {
         const size_t o = l * plane;
-        const float center = accum_load(A.fmt, A.shadow, o + pix);
-        float out;
-        if (A.frame > 0) {
-            const float old = accum_load(A.fmt, A.hist, o + pix);
-            const float a = __fdiv_rn(1.0f, __fadd_rn((float)A.frame, 1.0f));
-            out = __fadd_rn(__fmul_rn(old, __fsub_rn(1.0f, a)), __fmul_rn(center, a));
-        } else {
-            // blur.comp:53: the y term reuses the x motion (vec2(float, vec2) constructor)
-            const float lx = __fadd_rn((float)x, __fmul_rn(rx, (float)A.W));
-            const float ly = __fadd_rn((float)y, __fmul_rn(rx, (float)A.H));
-            float mn = center, mx = center;
-            for (int dy = -1; dy <= 1; dy++)
-                for (int dx = -1; dx <= 1; dx++) {
-                    if (dx == 0 && dy == 0) continue;
-                    int xx = (int)x + dx, yy = (int)y + dy;
-                    float c = 0.f;
-                    if (xx >= 0 && yy >= 0 && xx < (int)A.W && yy < (int)A.H)
-                        c = accum_load(A.fmt, A.shadow, o + (size_t)yy * A.W + xx);
-                    mn = fminf(mn, c);
-                    mx = fmaxf(mx, c);
-                }
-            float old = 0.f;
-            if (lx > -2147483648.f && lx < 2147483647.f && ly > -2147483648.f && ly < 2147483647.f) {
-                int ix = (int)lx, iy = (int)ly;
-                if (ix >= 0 && iy >= 0 && ix < (int)A.W && iy < (int)A.H)
-                    old = accum_load(A.fmt, A.hist_prev, o + (size_t)iy * A.W + ix);
-            }
-            old = fmaxf(mn, old);
-            old = fminf(mx, old);
-            out = __fadd_rn(__fmul_rn(old, __fsub_rn(1.0f, 0.4f)), __fmul_rn(center, 0.4f));
+        __syncthreads();  // the last light's tile has been read
+        for (uint32_t i = tid; i < (kBlurW + 2) * (kBlurH + 2); i += kBlurW * kBlurH) {
+            const uint32_t tx = i % (kBlurW + 2), ty = i / (kBlurW + 2);
+            const int xx = (int)(blockIdx.x * kBlurW + tx) - 1, yy = (int)(blockIdx.y * kBlurH + ty) - 1;
+            T c = 0;
+            if (xx >= 0 && yy >= 0 && xx < (int)A.W && yy < (int)A.H) c = raw[o + (size_t)yy * A.W + xx];
+            s_tile[ty][tx] = c;
         }
-        accum_store(A.fmt, A.hist, o + pix, out);
+        __syncthreads();
+        if (!present) continue;
+        const T mid = s_tile[ly + 1][lx + 1];
+        T lo = mid, hi = mid;
+#pragma unroll
+        for (int dy = 0; dy < 3; dy++)
+#pragma unroll
+            for (int dx = 0; dx < 3; dx++) {
+                if (dx == 1 && dy == 1) continue;
+                const T c = s_tile[ly + dy][lx + dx];
+                if constexpr (U8) { lo = c < lo ? c : lo; hi = c > hi ? c : hi; }
+                else { lo = fminf(lo, c); hi = fmaxf(hi, c); }
+            }
+        float old = inside ? value(prev[o + from]) : 0.f;
+        old = fmaxf(value(lo), old);
+        old = fminf(value(hi), old);
+        store(o + pix, __fadd_rn(__fmul_rn(old, __fsub_rn(1.0f, 0.4f)), __fmul_rn(value(mid), 0.4f)));
     }
 }
 
@@ -1126,9 +1167,10 @@ cudaError_t pixel_occupancy(int mode, bool count, int minb, bool two, bool short
 }
 
 cudaError_t launch_accumulate(const AccumParams& A, cudaStream_t s) {
-    dim3 b(16, 16), g((A.blur_w + 15) / 16, (A.blur_h + 15) / 16);
+    const dim3 g((A.blur_w + kBlurW - 1) / kBlurW, (A.blur_h + kBlurH - 1) / kBlurH);
     if (g.x == 0 || g.y == 0) return cudaSuccess;
-    k_accumulate<<<g, b, 0, s>>>(A);
+    if (A.fmt == HY_ACCUM_U8) k_accumulate<true><<<g, kBlurW * kBlurH, 0, s>>>(A);
+    else k_accumulate<false><<<g, kBlurW * kBlurH, 0, s>>>(A);
     return cudaGetLastError();
 }
 
