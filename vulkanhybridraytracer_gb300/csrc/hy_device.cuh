@@ -384,6 +384,16 @@ __device__ __forceinline__ unsigned long long f2_pack(float a, float b) {
 __device__ __forceinline__ void f2_unpack(unsigned long long v, float& a, float& b) {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
 }
+__device__ __forceinline__ unsigned long long f2_add(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ unsigned long long f2_mul(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
 __device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsigned long long b,
                                                      unsigned long long c) {
     unsigned long long d;
@@ -663,6 +673,8 @@ __device__ __forceinline__ bool trav_node(const SceneDev& S, const RW& rw, float
     // (NaN planes, 0 * inf, are skipped by max / min, and a difference with NaN
     // has a clear sign: such a box counts as hit, as with the comparisons.)
     const float tmaxc = __fmul_rn(t.tmax, kBoxSlack);
+    const unsigned long long slack2 = f2_pack(kBoxSlack, kBoxSlack), minus2 = f2_pack(-1.0f, -1.0f);
+    const unsigned long long tmax2 = f2_pack(tmaxc, tmaxc), tmin2 = f2_pack(-tmin, -tmin);
     uint32_t miss = 0;
 #pragma unroll
     for (int j = 3; j >= 0; j--) {  // slots 2j + 1, 2j: the funnel shift takes the highest slot first
@@ -675,14 +687,16 @@ __device__ __forceinline__ bool trav_node(const SceneDev& S, const RW& rw, float
             f2_unpack(f2_fma(f2_pack(n0, f0), adj2[a], org2[a]), tn[0][a], tf[0][a]);
             f2_unpack(f2_fma(f2_pack(n1, f1), adj2[a], org2[a]), tn[1][a], tf[1][a]);
         }
-#pragma unroll
-        for (int h = 1; h >= 0; h--) {
-            const float tnear = fmax3(tn[h][0], tn[h][1], tn[h][2]);
-            const float m = __fmul_rn(fmin3(tf[h][0], tf[h][1], tf[h][2]), kBoxSlack);
-            const uint32_t out = __float_as_uint(__fsub_rn(m, tnear)) | __float_as_uint(__fsub_rn(tmaxc, tnear)) |
-                                 __float_as_uint(__fsub_rn(m, tmin));
-            miss = __funnelshift_l(out, miss, 1);
-        }
+        // both slots' products and differences as f32x2 (tnear * -1 + m is m - tnear)
+        const unsigned long long near2 = f2_pack(fmax3(tn[0][0], tn[0][1], tn[0][2]), fmax3(tn[1][0], tn[1][1], tn[1][2]));
+        const unsigned long long m2 =
+            f2_mul(f2_pack(fmin3(tf[0][0], tf[0][1], tf[0][2]), fmin3(tf[1][0], tf[1][1], tf[1][2])), slack2);
+        float d0, d1, e0, e1, g0, g1;
+        f2_unpack(f2_fma(near2, minus2, m2), d0, d1);
+        f2_unpack(f2_fma(near2, minus2, tmax2), e0, e1);
+        f2_unpack(f2_add(m2, tmin2), g0, g1);
+        miss = __funnelshift_l(__float_as_uint(d1) | __float_as_uint(e1) | __float_as_uint(g1), miss, 1);
+        miss = __funnelshift_l(__float_as_uint(d0) | __float_as_uint(e0) | __float_as_uint(g0), miss, 1);
     }
     // internal children go to the stack in rank order, leaf slots give their
     // triangles (an empty slot, whose box is the node's lo corner, has none)
