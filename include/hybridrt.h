@@ -355,10 +355,13 @@ int hy_bvh_download_instances(HyCtx* ctx, float* records, float* boxes);
  *                        DRAM;
  *   HY_ANYHIT_AUTO       (default) far first for a one-level structure whose
  *                        nodes and leaf records fit in the device's L2, near
- *                        first otherwise (two-level structures included).
+ *                        first otherwise (two-level structures included); the
+ *                        default shadow schedule of an uncounted, unbatched
+ *                        pass takes far first for every one-level structure.
  * The order is a property of the scene: it applies to every pass on it,
  * batched views included.  hy_scene_anyhit_order reports the order a pass
- * uses now (HY_ERR_NOT_READY without a built structure).  Which triangle an
+ * uses now (HY_ERR_NOT_READY without a built structure; under AUTO the order
+ * of ray queries and counted passes).  Which triangle an
  * any-hit query reports can differ between the orders; whether it hits
  * cannot. */
 enum { HY_ANYHIT_AUTO = 0, HY_ANYHIT_FAR_FIRST = 1, HY_ANYHIT_NEAR_FIRST = 2 };

@@ -127,9 +127,10 @@ std::vector<float> normal_matrices(const float* xf, uint32_t n) {
 
 // HY_ANYHIT_AUTO: far first while the nodes (80 B) and leaf records (48 B)
 // fit in L2 — measured on a 1.5M-triangle scene (90 MB): 8.7 % fewer node
-// visits, 9.6 % faster; on a 7.35M-triangle one (440 MB): 26 % fewer visits
-// but 2 % slower, each visit's fetches going to DRAM — and near first for
-// two-level structures
+// visits, 9.6 % faster; on a 7.35M-triangle one (440 MB) the shade and
+// path-trace kernels are 5 % and 2 % slower so, each visit's fetches going to
+// DRAM — and near first for two-level structures.  stream_scene() has the
+// tile-stream shadow kernel's rule.
 static uint32_t anyhit_flip(const HyCtx* c) {
     if (c->anyhit_order == HY_ANYHIT_FAR_FIRST) return 7u;
     if (c->anyhit_order == HY_ANYHIT_NEAR_FIRST || c->two_level) return 0u;
@@ -346,6 +347,20 @@ struct ProfScope {
     }
 };
 
+// The scene of a tile-stream shadow launch.  HY_ANYHIT_AUTO walks every one-level
+// structure far first here, also one beyond L2: the kernel keeps enough walks in
+// flight per SM for the fewer visits to pay although their fetches go to DRAM
+// (far / near, 7.3M triangles in 440 MB: 4K with 64 lights, one ray each, 105.2 /
+// 123.9 ms; 1080p with 16 lights 6.85 / 7.47, with 4 samples 18.5 / 20.8).  The shade
+// (3.70 / 3.51) and path-trace (7.55 / 7.39) kernels there and two-level structures
+// (10 MB of instance records and 1,025 instances 12.8 / 10.9) keep their order.  Counted
+// passes walk in the order that hy_scene_anyhit_order reports.
+static SceneDev stream_scene(HyCtx* c, bool count) {
+    SceneDev S = scene_dev(c);
+    if (c->anyhit_order == HY_ANYHIT_AUTO && !count && !c->two_level) S.anyhit_flip = 7u;
+    return S;
+}
+
 int run_pixels(HyCtx* c, int mode, const PassParams& P0, const HyPassConfig* cfg, int queue_slot) {
     bool count = (cfg->flags & HY_FLAG_COUNT_TRAVERSAL) != 0;
     int block = cfg->block_size ? (int)cfg->block_size : 128;
@@ -409,7 +424,8 @@ int run_pixels(HyCtx* c, int mode, const PassParams& P0, const HyPassConfig* cfg
     }
     grid = std::max(1, std::min<int>(grid, (int)((P.units * 32ull + block - 1) / block)));
     ProfScope prof(c, mode);
-    HY_CUDA_TRY(launch_pixels(mode, count, minb, scene_dev(c), P, grid, block, c->stream));
+    HY_CUDA_TRY(launch_pixels(mode, count, minb, streams ? stream_scene(c, count) : scene_dev(c), P, grid, block,
+                              c->stream));
     return HY_OK;
 }
 
