@@ -10,9 +10,9 @@
 //   k_karras        Karras 2012 binary radix tree over (morton << 32 | id)
 //                   (HY_BUILD_LBVH), or the binned-SAH tree of hy_sah.cu
 //                   over the same order (HY_BUILD_SAH, the default)
-//   k_boxes_dp      bottom-up boxes and the slot budgets of the collapse by the surface
-//                   area heuristic, last arriver computes (no waiting); k_refit: the
-//                   boxes alone
+//   k_climb         bottom-up boxes and the slot budgets of the collapse by the surface
+//                   area heuristic (a refit: the boxes alone), by blocks of leaves in
+//                   shared memory, above them last arriver computes (no waiting)
 //   k_collapse_*    BFS collapse into compressed 8-wide nodes, one level per
 //                   launch pair with prefix sums for deterministic numbering
 //
@@ -409,27 +409,6 @@ __device__ __forceinline__ void child_box(uint32_t c, const uint32_t* bvh2, cons
     }
 }
 
-__global__ void k_refit(const uint32_t* __restrict__ order, const float* __restrict__ tribox, uint32_t n,
-                        uint32_t* bvh2, const uint32_t* __restrict__ parent, uint32_t* flags) {
-    uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    uint32_t p = parent[n - 1 + j];
-    while (p != 0xffffffffu) {
-        __threadfence();
-        if (atomicAdd(flags + p, 1u) == 0u) return;  // the sibling's thread finishes this node
-        __threadfence();
-        uint32_t* nd = bvh2 + (size_t)p * 10;
-        float l0[3], h0[3], l1[3], h1[3];
-        child_box(__ldcg(nd + 0), bvh2, order, tribox, l0, h0);
-        child_box(__ldcg(nd + 1), bvh2, order, tribox, l1, h1);
-        for (int a = 0; a < 3; a++) {
-            __stcg(nd + 4 + a, __float_as_uint(fminf(l0[a], l1[a])));
-            __stcg(nd + 7 + a, __float_as_uint(fmaxf(h0[a], h1[a])));
-        }
-        p = parent[p];
-    }
-}
-
 // ---------------------------------------------------------------------------------
 // BVH8 collapse
 // ---------------------------------------------------------------------------------
@@ -465,20 +444,56 @@ __device__ __forceinline__ float surface(const Ref& b) {
 // (a leaf slot of <= kLeafMax triangles: area x triangles x kCostTri; an
 // internal node: area x kCostNode + its own 8 slots); a one-triangle leaf
 // costs area x kCostTri.  dpk[n * 9]: left share k of the node's own 8 slots;
-// dpk[n * 9 + i]: the left share of i slots, 0 for "i - 1 slots".  The second
-// child to finish computes its parent (as k_refit), reading the first's
-// values through L2; the float ops and tie rule (first strict minimum in k
-// order) are the oracle's.
+// dpk[n * 9 + i]: the left share of i slots, 0 for "i - 1 slots".  The float ops
+// and tie rule (first strict minimum in k order) are the oracle's.
 constexpr float kCostNode = 1.0f, kCostTri = 0.5f;
 
-// The boxes of the binary tree (as k_refit) and the slot budgets in one climb.
-__device__ __forceinline__ void dp_child(uint32_t m, const float lo[3], const float hi[3], const float* dpf, float f[8]) {
-    if (m & kLeaf) {
-        Ref b;
-        for (int a = 0; a < 3; a++) { b.lo[a] = lo[a]; b.hi[a] = hi[a]; }
-        const float v = __fmul_rn(surface(b), kCostTri);
+__device__ __forceinline__ void leaf_budgets(const float lo[3], const float hi[3], float f[8]) {
+    Ref b;
+    for (int a = 0; a < 3; a++) { b.lo[a] = lo[a]; b.hi[a] = hi[a]; }
+    const float v = __fmul_rn(surface(b), kCostTri);
 #pragma unroll
-        for (int i = 0; i < 8; i++) f[i] = v;
+    for (int i = 0; i < 8; i++) f[i] = v;
+}
+
+// a node's costs f from its children's; returns its choices, 3 bits each: dpk[0], dpk[2..8]
+__device__ __forceinline__ uint32_t slot_budgets(const Ref& nb, const float fl[8], const float fr[8], float f[8]) {
+    const float A = surface(nb);
+    float best8 = INFINITY;
+    int bk = 1;
+#pragma unroll
+    for (int k = 1; k <= 7; k++) {
+        const float v = __fadd_rn(fl[k - 1], fr[8 - k - 1]);
+        if (v < best8) { best8 = v; bk = k; }
+    }
+    f[0] = nb.count <= (uint32_t)kLeafMax ? __fmul_rn(__fmul_rn(A, __uint2float_rn(nb.count)), kCostTri)
+                                          : __fadd_rn(__fmul_rn(A, kCostNode), best8);
+    uint32_t ks = (uint32_t)bk;
+#pragma unroll
+    for (int i = 2; i <= 8; i++) {
+        float v = f[i - 2];
+        int kk = 0;
+#pragma unroll
+        for (int k = 1; k < i; k++) {
+            const float w = __fadd_rn(fl[k - 1], fr[i - k - 1]);
+            if (w < v) { v = w; kk = k; }
+        }
+        f[i - 1] = v;
+        ks |= (uint32_t)kk << (3 * (i - 1));
+    }
+    return ks;
+}
+
+__device__ __forceinline__ void store_choices(uint8_t* kd, uint32_t ks) {
+    kd[0] = (uint8_t)(ks & 7u);
+#pragma unroll
+    for (int i = 2; i <= 8; i++) kd[i] = (uint8_t)((ks >> (3 * (i - 1))) & 7u);
+}
+
+__device__ __forceinline__ void child_budgets(uint32_t m, const float lo[3], const float hi[3], const float* dpf,
+                                              float f[8]) {
+    if (m & kLeaf) {
+        leaf_budgets(lo, hi, f);
     } else {
         const float4 p = __ldcg((const float4*)(dpf + (size_t)m * 8)), q = __ldcg((const float4*)(dpf + (size_t)m * 8) + 1);
         f[0] = p.x; f[1] = p.y; f[2] = p.z; f[3] = p.w;
@@ -486,63 +501,149 @@ __device__ __forceinline__ void dp_child(uint32_t m, const float lo[3], const fl
     }
 }
 
-__global__ void k_boxes_dp(const uint32_t* __restrict__ order, const float* __restrict__ tribox, uint32_t n,
-                           uint32_t* bvh2, const uint32_t* __restrict__ parent, uint32_t* flags, float* dpf,
-                           uint8_t* dpk) {
-    uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    uint32_t p = parent[n - 1 + j];
+// The boxes of the binary tree and, with DP, the slot budgets, bottom up.  A block takes
+// kClimb consecutive leaves.  A node's index lies within its range in both trees, so the
+// nodes whose range lies in the block's leaves sit in the block's slots: they are read and
+// written as coalesced runs and climbed in shared memory, in rounds over the nodes whose
+// children are done.  What leaves the block goes up through global flags: the second child
+// to finish computes its parent, reading the first's values through L2.
+// Bound by the latency of the climb above the blocks; a node's topology is read while the
+// sibling may still be at work (with the budgets 224 us read after the flag).  With every
+// node through global flags (two atomics and two device fences a node, ever fewer live
+// lanes) 1.5M triangles took 175 us for the boxes alone and 590 with the budgets, now 128
+// and 208; blocks of 512: 149 for the boxes (139 with 256, both read after the flag).
+constexpr uint32_t kClimb = 256;
+
+template <bool DP>
+__global__ void __launch_bounds__(kClimb) k_climb(const uint32_t* __restrict__ order,
+                                                  const float* __restrict__ tribox, uint32_t n, uint32_t* bvh2,
+                                                  const uint32_t* __restrict__ parent, uint32_t* flags, float* dpf,
+                                                  uint8_t* dpk) {
+    __shared__ float s_box[6][2 * kClimb];  // leaf i at i, node slot i at kClimb + i
+    __shared__ uint32_t s_left[kClimb], s_right[kClimb], s_up[kClimb], s_count[kClimb], s_flag[kClimb];
+    __shared__ uint16_t s_ready[kClimb];
+    __shared__ uint32_t s_out[kClimb];  // parents outside the block, one per subtree (at most one per leaf)
+    __shared__ float s_f[DP ? 8 : 1][DP ? kClimb : 1];
+    __shared__ uint32_t s_k[DP ? kClimb : 1];
+    __shared__ uint32_t s_nready, s_nout;
+    const uint32_t t = threadIdx.x, base = blockIdx.x * kClimb, j = base + t, end = min(n, base + kClimb);
+    uint32_t leaf_up = 0xffffffffu;
+    s_count[t] = 0;  // 0: not a node of this block
+    s_flag[t] = 0;
+    if (t == 0) s_nready = s_nout = 0;
+    if (j < n - 1) {
+        const uint2* nd = (const uint2*)(bvh2 + (size_t)j * 10);
+        const uint2 lr = nd[0], fl = nd[1];
+        if (fl.x >= base && fl.y < end) {
+            s_left[t] = lr.x;
+            s_right[t] = lr.y;
+            s_up[t] = parent[j];
+            s_count[t] = fl.y - fl.x + 1;
+        }
+    }
+    if (j < n) {
+        const float2* b = (const float2*)(tribox + (size_t)order[j] * 6);
+        const float2 x = b[0], y = b[1], z = b[2];
+        s_box[0][t] = x.x; s_box[1][t] = x.y; s_box[2][t] = y.x;
+        s_box[3][t] = y.y; s_box[4][t] = z.x; s_box[5][t] = z.y;
+        leaf_up = parent[n - 1 + j];
+    }
+    __syncthreads();
+    // one child of node p is done; true: p is now ready
+    auto arrive = [&](uint32_t p) -> bool {
+        if (p == 0xffffffffu) return false;
+        const uint32_t i = p - base;
+        if (i >= kClimb || !s_count[i]) {
+            s_out[atomicAdd(&s_nout, 1u)] = p;
+            return false;
+        }
+        if (atomicAdd(&s_flag[i], 1u) == 0u) return false;
+        s_ready[atomicAdd(&s_nready, 1u)] = (uint16_t)i;
+        return true;
+    };
+    uint32_t done = 0, avail = (uint32_t)__syncthreads_count(j < n && arrive(leaf_up));
+    while (done < avail) {  // each thread pushes at most one node a round: the count ends the round
+        bool pushed = false;
+        if (done + t < avail) {
+            const uint32_t i = s_ready[done + t];
+            Ref nb;
+            nb.count = s_count[i];
+            const uint32_t L = s_left[i], R = s_right[i];
+            const uint32_t l = (L & kLeaf) ? (L & ~kLeaf) - base : kClimb + L - base;
+            const uint32_t r = (R & kLeaf) ? (R & ~kLeaf) - base : kClimb + R - base;
+            float l0[3], h0[3], l1[3], h1[3];
+#pragma unroll
+            for (int a = 0; a < 3; a++) {
+                l0[a] = s_box[a][l]; h0[a] = s_box[3 + a][l];
+                l1[a] = s_box[a][r]; h1[a] = s_box[3 + a][r];
+                s_box[a][kClimb + i] = nb.lo[a] = fminf(l0[a], l1[a]);
+                s_box[3 + a][kClimb + i] = nb.hi[a] = fmaxf(h0[a], h1[a]);
+            }
+            if (DP) {
+                float fl[8], fr[8], f[8];
+                if (L & kLeaf) leaf_budgets(l0, h0, fl);
+                else
+#pragma unroll
+                    for (int a = 0; a < 8; a++) fl[a] = s_f[a][l - kClimb];
+                if (R & kLeaf) leaf_budgets(l1, h1, fr);
+                else
+#pragma unroll
+                    for (int a = 0; a < 8; a++) fr[a] = s_f[a][r - kClimb];
+                s_k[i] = slot_budgets(nb, fl, fr, f);
+#pragma unroll
+                for (int a = 0; a < 8; a++) s_f[a][i] = f[a];
+            }
+            pushed = arrive(s_up[i]);
+        }
+        done = avail;
+        avail += (uint32_t)__syncthreads_count(pushed);
+    }
+    if (s_count[t]) {
+        uint2* nd = (uint2*)(bvh2 + (size_t)j * 10 + 4);
+#pragma unroll
+        for (int a = 0; a < 3; a++)
+            __stcg(nd + a, make_uint2(__float_as_uint(s_box[2 * a][kClimb + t]),
+                                      __float_as_uint(s_box[2 * a + 1][kClimb + t])));
+        if (DP) {
+            store_choices(dpk + (size_t)j * 9, s_k[t]);
+            const uint32_t i = s_up[t] - base;
+            if (i >= kClimb || !s_count[i]) {  // read by a parent outside the block
+                float4* fo = (float4*)(dpf + (size_t)j * 8);
+                __stcg(fo, make_float4(s_f[0][t], s_f[1][t], s_f[2][t], s_f[3][t]));
+                __stcg(fo + 1, make_float4(s_f[4][t], s_f[5][t], s_f[6][t], s_f[7][t]));
+            }
+        }
+    }
+    __syncthreads();
+    if (t >= s_nout) return;
+    uint32_t p = s_out[t];
     while (p != 0xffffffffu) {
+        uint32_t* nd = bvh2 + (size_t)p * 10;
+        const uint2 lr = *(const uint2*)nd, fl = *(const uint2*)(nd + 2);
+        const uint32_t L = lr.x, R = lr.y, up = parent[p];
+        Ref nb;
+        nb.count = fl.y - fl.x + 1;
         __threadfence();
         if (atomicAdd(flags + p, 1u) == 0u) return;  // the sibling's thread computes this node
         __threadfence();
-        uint32_t* nd = bvh2 + (size_t)p * 10;
-        const uint32_t L = __ldcg(nd + 0), R = __ldcg(nd + 1), first = __ldcg(nd + 2), last = __ldcg(nd + 3);
-        const uint32_t up = parent[p];
-        Ref nb;
-        float fl[8], fr[8];
-        {
-            float l0[3], h0[3], l1[3], h1[3];
-            child_box(L, bvh2, order, tribox, l0, h0);
-            child_box(R, bvh2, order, tribox, l1, h1);
-            dp_child(L, l0, h0, dpf, fl);
-            dp_child(R, l1, h1, dpf, fr);
-            for (int a = 0; a < 3; a++) {
-                nb.lo[a] = fminf(l0[a], l1[a]);
-                nb.hi[a] = fmaxf(h0[a], h1[a]);
-                __stcg(nd + 4 + a, __float_as_uint(nb.lo[a]));
-                __stcg(nd + 7 + a, __float_as_uint(nb.hi[a]));
-            }
+        float l0[3], h0[3], l1[3], h1[3];
+        child_box(L, bvh2, order, tribox, l0, h0);
+        child_box(R, bvh2, order, tribox, l1, h1);
+        for (int a = 0; a < 3; a++) {
+            nb.lo[a] = fminf(l0[a], l1[a]);
+            nb.hi[a] = fmaxf(h0[a], h1[a]);
+            __stcg(nd + 4 + a, __float_as_uint(nb.lo[a]));
+            __stcg(nd + 7 + a, __float_as_uint(nb.hi[a]));
         }
-        const float A = surface(nb);
-        const uint32_t cnt = last - first + 1;
-        float best8 = INFINITY;
-        int bk = 1;
-#pragma unroll
-        for (int k = 1; k <= 7; k++) {
-            const float v = __fadd_rn(fl[k - 1], fr[8 - k - 1]);
-            if (v < best8) { best8 = v; bk = k; }
+        if (DP) {
+            float fl[8], fr[8], f[8];
+            child_budgets(L, l0, h0, dpf, fl);
+            child_budgets(R, l1, h1, dpf, fr);
+            store_choices(dpk + (size_t)p * 9, slot_budgets(nb, fl, fr, f));
+            float4* fo = (float4*)(dpf + (size_t)p * 8);
+            __stcg(fo, make_float4(f[0], f[1], f[2], f[3]));
+            __stcg(fo + 1, make_float4(f[4], f[5], f[6], f[7]));
         }
-        float f[8];
-        f[0] = cnt <= (uint32_t)kLeafMax ? __fmul_rn(__fmul_rn(A, __uint2float_rn(cnt)), kCostTri)
-                                         : __fadd_rn(__fmul_rn(A, kCostNode), best8);
-        uint8_t* kd = dpk + (size_t)p * 9;
-        kd[0] = (uint8_t)bk;
-#pragma unroll
-        for (int i = 2; i <= 8; i++) {
-            float v = f[i - 2];
-            int kk = 0;
-#pragma unroll
-            for (int k = 1; k < i; k++) {
-                const float w = __fadd_rn(fl[k - 1], fr[i - k - 1]);
-                if (w < v) { v = w; kk = k; }
-            }
-            f[i - 1] = v;
-            kd[i] = (uint8_t)kk;
-        }
-        float4* fo = (float4*)(dpf + (size_t)p * 8);
-        __stcg(fo, make_float4(f[0], f[1], f[2], f[3]));
-        __stcg(fo + 1, make_float4(f[4], f[5], f[6], f[7]));
         p = up;
     }
 }
@@ -851,9 +952,9 @@ static int build_core(HyCtx* c, uint32_t n, uint32_t node_off, uint32_t rec_off,
             k_karras<<<cdiv(n - 1, 256), 256, 0, s>>>(mort, ord, n, bvh2, c->parent.as<uint32_t>());
         }
         HY_CUDA_TRY(cudaMemsetAsync(c->flags.p, 0, (size_t)n * 4, s));
-        k_boxes_dp<<<cdiv(n, 256), 256, 0, s>>>(ord, c->tribox.as<float>(), n, bvh2, c->parent.as<uint32_t>(),
-                                                c->flags.as<uint32_t>(), c->dp_cost.as<float>(),
-                                                c->dp_k.as<uint8_t>());
+        k_climb<true><<<cdiv(n, kClimb), kClimb, 0, s>>>(ord, c->tribox.as<float>(), n, bvh2,
+                                                         c->parent.as<uint32_t>(), c->flags.as<uint32_t>(),
+                                                         c->dp_cost.as<float>(), c->dp_k.as<uint8_t>());
     }
     HY_CUDA_TRY(cudaGetLastError());
     uint32_t level_start = 0, tri_start = 0, m = 1, depth = 0;
@@ -945,9 +1046,9 @@ int bvh_refit_impl(HyCtx* c) {
     if ((rc = world_tris_impl(c))) return rc;
     if (n > 1) {
         HY_CUDA_TRY(cudaMemsetAsync(c->flags.p, 0, (size_t)n * 4, s));
-        k_refit<<<cdiv(n, 256), 256, 0, s>>>(c->vals[0].as<uint32_t>(), c->tribox.as<float>(), n,
-                                             c->bvh2.as<uint32_t>(), c->parent.as<uint32_t>(),
-                                             c->flags.as<uint32_t>());
+        k_climb<false><<<cdiv(n, kClimb), kClimb, 0, s>>>(c->vals[0].as<uint32_t>(), c->tribox.as<float>(), n,
+                                                          c->bvh2.as<uint32_t>(), c->parent.as<uint32_t>(),
+                                                          c->flags.as<uint32_t>(), nullptr, nullptr);
     }
     k_requantize<<<cdiv(c->n_bvh8, 128), 128, 0, s>>>(c->n_bvh8, c->node_ref.as<uint32_t>(),
                                                       c->node_plan.as<uint32_t>(), c->bvh2.as<uint32_t>(),
