@@ -37,17 +37,18 @@ __device__ __forceinline__ int f2ord(float f) {
 __device__ __forceinline__ float ord2f(int i) { return __int_as_float(i >= 0 ? i : i ^ 0x7fffffff); }
 
 // ---------------------------------------------------------------------------------
-__global__ void k_world_tris(const HyVertex* __restrict__ verts, const uint32_t* __restrict__ idx,
-                             const HyPrimitive* __restrict__ prims, const uint32_t* __restrict__ tri_prim,
-                             const uint32_t* __restrict__ prim_tri0, const float* __restrict__ xf, uint32_t n,
-                             float4* __restrict__ world, float* __restrict__ tribox, float4* __restrict__ cen) {
-    uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
+// triangle t's world vertices (w = 0) and box
+__device__ __forceinline__ void world_triangle(const HyVertex* __restrict__ verts, const uint32_t* __restrict__ idx,
+                                               const HyPrimitive* __restrict__ prims,
+                                               const uint32_t* __restrict__ tri_prim,
+                                               const uint32_t* __restrict__ prim_tri0, const float* __restrict__ xf,
+                                               uint32_t t, float4 out[3], float lo[3], float hi[3]) {
     uint32_t p = tri_prim[t];
     HyPrimitive pr = prims[p];
     uint32_t local = t - prim_tri0[p];
     const float* M = xf + (size_t)pr.transform_id * 16;
-    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    for (int a = 0; a < 3; a++) { lo[a] = INFINITY; hi[a] = -INFINITY; }
+#pragma unroll
     for (int v = 0; v < 3; v++) {
         uint32_t vi = idx[pr.first_index + 3 * local + v] + pr.vertex_offset;
         const float* P = verts[vi].pos;
@@ -62,8 +63,20 @@ __global__ void k_world_tris(const HyVertex* __restrict__ verts, const uint32_t*
             lo[r] = fminf(lo[r], acc);
             hi[r] = fmaxf(hi[r], acc);
         }
-        world[(size_t)t * 3 + v] = make_float4(w[0], w[1], w[2], 0.f);
+        out[v] = make_float4(w[0], w[1], w[2], 0.f);
     }
+}
+
+__global__ void k_world_tris(const HyVertex* __restrict__ verts, const uint32_t* __restrict__ idx,
+                             const HyPrimitive* __restrict__ prims, const uint32_t* __restrict__ tri_prim,
+                             const uint32_t* __restrict__ prim_tri0, const float* __restrict__ xf, uint32_t n,
+                             float4* __restrict__ world, float* __restrict__ tribox, float4* __restrict__ cen) {
+    uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    float4 w[3];
+    float lo[3], hi[3];
+    world_triangle(verts, idx, prims, tri_prim, prim_tri0, xf, t, w, lo, hi);
+    for (int v = 0; v < 3; v++) world[(size_t)t * 3 + v] = w[v];
     float* b = tribox + (size_t)t * 6;
     for (int a = 0; a < 3; a++) { b[a] = lo[a]; b[3 + a] = hi[a]; }
     cen[t] = make_float4(__fmul_rn(__fadd_rn(lo[0], hi[0]), 0.5f), __fmul_rn(__fadd_rn(lo[1], hi[1]), 0.5f),
@@ -858,17 +871,27 @@ __global__ void k_requantize(uint32_t n_nodes, const uint32_t* __restrict__ node
     for (int a = 0; a < 3; a++) nd.q[2 + a] = make_uint4(q[a][0], q[a][1], q[a][2], q[a][3]);
 }
 
-// packed triangles take their (new) world vertices by the id they carry
-__global__ void k_repack_tris(uint32_t n, const float4* __restrict__ world, float4* __restrict__ tris) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+// Refit: each packed triangle takes its new world vertices by the id it carries, and
+// its box is written for the climb (as k_world_tris).  Bound by the gathers of the vertices:
+// 64 us for 1.5M triangles, against 52 for all triangles' vertices, boxes and centroids
+// and 41 for packing them again.
+__global__ void k_refit_tris(const HyVertex* __restrict__ verts, const uint32_t* __restrict__ idx,
+                             const HyPrimitive* __restrict__ prims, const uint32_t* __restrict__ tri_prim,
+                             const uint32_t* __restrict__ prim_tri0, const float* __restrict__ xf, uint32_t n,
+                             float4* __restrict__ tris, float* __restrict__ tribox) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float4* t = tris + (size_t)i * 3;
     const uint32_t id = __float_as_uint(t[0].w);
-    float4 v0 = world[(size_t)id * 3], v1 = world[(size_t)id * 3 + 1], v2 = world[(size_t)id * 3 + 2];
-    v0.w = __uint_as_float(id);
-    v1.w = 0.f;
-    v2.w = 0.f;
-    t[0] = v0; t[1] = v1; t[2] = v2;
+    float4 w[3];
+    float lo[3], hi[3];
+    world_triangle(verts, idx, prims, tri_prim, prim_tri0, xf, id, w, lo, hi);
+    w[0].w = __uint_as_float(id);
+    t[0] = w[0]; t[1] = w[1]; t[2] = w[2];
+    float2* b = (float2*)(tribox + (size_t)id * 6);
+    b[0] = make_float2(lo[0], lo[1]);
+    b[1] = make_float2(lo[2], hi[0]);
+    b[2] = make_float2(hi[1], hi[2]);
 }
 
 // ---------------------------------------------------------------------------------
@@ -1043,7 +1066,11 @@ int bvh_refit_impl(HyCtx* c) {
     const uint32_t n = c->ntri;
     int rc;
     cudaStream_t s = c->stream;
-    if ((rc = world_tris_impl(c))) return rc;
+    if ((rc = ctx_alloc(c, c->tribox, (size_t)n * 24))) return rc;
+    k_refit_tris<<<cdiv(n, 256), 256, 0, s>>>(c->verts.as<HyVertex>(), c->idx.as<uint32_t>(),
+                                              c->prims.as<HyPrimitive>(), c->tri_prim.as<uint32_t>(),
+                                              c->prim_tri0.as<uint32_t>(), c->xf.as<float>(), n, c->tris.as<float4>(),
+                                              c->tribox.as<float>());
     if (n > 1) {
         HY_CUDA_TRY(cudaMemsetAsync(c->flags.p, 0, (size_t)n * 4, s));
         k_climb<false><<<cdiv(n, kClimb), kClimb, 0, s>>>(c->vals[0].as<uint32_t>(), c->tribox.as<float>(), n,
@@ -1054,7 +1081,6 @@ int bvh_refit_impl(HyCtx* c) {
                                                       c->node_plan.as<uint32_t>(), c->bvh2.as<uint32_t>(),
                                                       c->vals[0].as<uint32_t>(), c->tribox.as<float>(),
                                                       c->nodes.as<Node8>());
-    k_repack_tris<<<cdiv(n, 256), 256, 0, s>>>(n, c->world.as<float4>(), c->tris.as<float4>());
     HY_CUDA_TRY(cudaGetLastError());
     HY_CUDA_TRY(cudaStreamSynchronize(s));
     return HY_OK;
