@@ -202,7 +202,7 @@ typedef struct HyPassConfig {
                                0 = 6 for the lane-group kernel, 8 otherwise */
     uint32_t visits_per_round; /* BVH node visits a shadow lane makes between two scheduling rounds
                                   of the persistent shadow kernels (1..16; a lane whose ray ends
-                                  early waits for the round); 0 = 4 */
+                                  early waits for the round); 0 = 4, 32 in counting launches */
 } HyPassConfig;
 
 typedef struct HyStats {

@@ -262,7 +262,11 @@ int grid_for(HyCtx* c, int mode, bool count, int minb, bool short_stack, int sha
 // walking on behind an occluder: shadow kernel at 3 / 4 / 6 / 8 / 12 visits, 1080p x
 // 16 spp 18.25 / 17.88 / 17.83 / 17.86 / 18.23 ms, 4K x 64 lights 144.1 / 143.1 /
 // 146.6 / 149.2 / 161.0 ms, 1277x719 two-level 13.5 / 13.0 / 13.0 / 13.2 / 13.7 ms
-constexpr uint32_t kStreamSteps = 4;
+// A counting launch tests each node's triangles at once (its counts are the plain walk's),
+// so a round's end is a cost alone there: rounds of 32 (counting shadow kernel at 4 / 16 /
+// 32 visits: 1080p 26.0 / 21.8 / 20.6 ms, two-level 16.8 / 16.0 / 13.6, path trace 5.5 / 4.9 / 4.7).
+constexpr uint32_t kStreamSteps = 4, kCountSteps = 32;
+inline uint32_t stream_steps(bool count) { return count ? kCountSteps : kStreamSteps; }
 
 PassParams make_params(HyCtx* c, const HyGBuffer* gb, const HyCamera* cam, const HyPassConfig* cfg,
                        uint32_t accum_fmt, void* shadow, void* hist, float* out_f, uint8_t* out_8) {
@@ -395,7 +399,7 @@ int run_pixels(HyCtx* c, int mode, const PassParams& P0, const HyPassConfig* cfg
     const bool grouped = mode == MODE_SHADOW_G || mode == MODE_SHADOW_ACCUM_G;
     const bool streams = mode >= MODE_SHADOW_S;
     int minb = cfg->min_blocks ? (int)cfg->min_blocks : (grouped ? 6 : 8);
-    if (streams && !cfg->visits_per_round) P.inner = kStreamSteps;
+    if (streams && !cfg->visits_per_round) P.inner = stream_steps(count);
     if (cfg->stack_depth && cfg->stack_depth != 8) return HY_ERR_UNSUPPORTED;
     P.short_stack = streams && !c->two_level && cfg->stack_depth == 8;
     // the shade kernel at 8 resident blocks (64 registers): 1.69 ms per 1080p frame
@@ -980,7 +984,7 @@ int hy_pathtrace_pass(HyCtx* c, const HyCamera* cam, uint32_t W, uint32_t H, con
     const bool count = (cfg->flags & HY_FLAG_COUNT_TRAVERSAL) != 0;
     // shadow rays of each hit as tile streams (default), or on the hit's own lane
     const bool stream = !(cfg->flags & HY_FLAG_PIXEL_PARALLEL);
-    P.inner = cfg->visits_per_round ? std::min(cfg->visits_per_round, 16u) : kStreamSteps;
+    P.inner = cfg->visits_per_round ? std::min(cfg->visits_per_round, 16u) : stream_steps(count);
     // resident blocks the tile-stream kernel is compiled for: 6 (80 registers)
     // measured fastest at 1080p (uncapped 195 registers: 1,015; 3: 1,351; 4: 1,536;
     // 5: 1,697; 6: 1,769; 8: 1,774 Mrays/s) — occupancy beats the spills
@@ -1195,7 +1199,7 @@ int hy_batch_forward(HyCtx* c, HyCtx* const* scenes, uint32_t ns, const HyView* 
                             v.out_rgba32f, v.out_bgra8);
         pv[i].scene = v.scene;
         pv[i].num_lights = v.accum.num_lights;
-        if (stream && !v.config.visits_per_round) pv[i].inner = kStreamSteps;
+        if (stream && !v.config.visits_per_round) pv[i].inner = stream_steps(count);
         uint32_t G = 1;
         if (v.config.rng_mode == HY_RNG_DECORRELATED)
             while (G < v.config.shadow_spp && G < 32) G <<= 1;
