@@ -389,11 +389,6 @@ __device__ __forceinline__ unsigned long long f2_add(unsigned long long a, unsig
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
-__device__ __forceinline__ unsigned long long f2_mul(unsigned long long a, unsigned long long b) {
-    unsigned long long d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
 __device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsigned long long b,
                                                      unsigned long long c) {
     unsigned long long d;
@@ -667,13 +662,17 @@ __device__ __forceinline__ bool trav_node(const SceneDev& S, const RW& rw, float
     const uint32_t q[3][4] = {{q2.x, q2.y, q2.z, q2.w}, {q3.x, q3.y, q3.z, q3.w}, {q4.x, q4.y, q4.z, q4.w}};
     // A box is hit when max(tn, tmin) <= rn(min(tf, tmax) * c).  rn(. * c) is
     // monotone, so that is tn <= rn(tf c), tn <= rn(tmax c), tmin <= rn(tf c) (a
-    // ray has tmin <= tmax): three differences whose signs are exact, gathered by one
-    // three-input OR and one funnel shift per slot.  The differences run on the FMA
-    // pipe; min / max / compare would run on the ALU pipe, which limits the walk.
+    // ray has tmin <= tmax): three differences, product minus left-hand side, whose
+    // sign bits are gathered by one three-input OR and one funnel shift per slot.
+    // The differences run on the FMA pipe; min / max / compare would run on the ALU
+    // pipe, which limits the walk.  Terms that differ give a difference of the right
+    // sign, equal ones +0, except (-0) - (+0) = -0: the products are fmas with +0, which
+    // make +0 of the -0 of a plane or an interval's end at the ray's origin.
     // (NaN planes, 0 * inf, are skipped by max / min, and a difference with NaN
     // has a clear sign: such a box counts as hit, as with the comparisons.)
-    const float tmaxc = __fmul_rn(t.tmax, kBoxSlack);
+    const float tmaxc = __fmaf_rn(t.tmax, kBoxSlack, 0.f);
     const unsigned long long slack2 = f2_pack(kBoxSlack, kBoxSlack), minus2 = f2_pack(-1.0f, -1.0f);
+    const unsigned long long zero2 = f2_pack(0.f, 0.f);
     const unsigned long long tmax2 = f2_pack(tmaxc, tmaxc), tmin2 = f2_pack(-tmin, -tmin);
     uint32_t miss = 0;
 #pragma unroll
@@ -689,8 +688,8 @@ __device__ __forceinline__ bool trav_node(const SceneDev& S, const RW& rw, float
         }
         // both slots' products and differences as f32x2 (tnear * -1 + m is m - tnear)
         const unsigned long long near2 = f2_pack(fmax3(tn[0][0], tn[0][1], tn[0][2]), fmax3(tn[1][0], tn[1][1], tn[1][2]));
-        const unsigned long long m2 =
-            f2_mul(f2_pack(fmin3(tf[0][0], tf[0][1], tf[0][2]), fmin3(tf[1][0], tf[1][1], tf[1][2])), slack2);
+        const unsigned long long m2 = f2_fma(
+            f2_pack(fmin3(tf[0][0], tf[0][1], tf[0][2]), fmin3(tf[1][0], tf[1][1], tf[1][2])), slack2, zero2);
         float d0, d1, e0, e1, g0, g1;
         f2_unpack(f2_fma(near2, minus2, m2), d0, d1);
         f2_unpack(f2_fma(near2, minus2, tmax2), e0, e1);
