@@ -4,6 +4,7 @@
 
 namespace hy {
 void* stream_kernel_accum(bool count, int minb, bool short_stack, bool one) {
-    return stream_kernel_flat<true>(count, minb, short_stack, one);
+    return one ? stream_kernel_flat<true, true>(count, minb, short_stack)
+               : stream_kernel_flat<true, false>(count, minb, short_stack);
 }
 }  // namespace hy

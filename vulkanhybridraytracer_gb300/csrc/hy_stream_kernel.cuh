@@ -72,34 +72,41 @@ __global__ void __launch_bounds__(128, MINB) k_shadow_stream(const SceneDev S, c
             l0 = part * P.part_lights;
             l1 = min(l0 + P.part_lights, P.num_lights);
         }
-        if constexpr (ONE)
-            stream_tile_one<COUNT, TWO, ACCUM ? 1 : 0>(S, P, tile, l0, l1, reference, ACCUM, sm.warp[threadIdx.x >> 5],
-                                                       stk, t, r, s, ls, nn, nt);
-        else if constexpr (SHORT)
-            stream_tile<COUNT, TWO, ACCUM ? 1 : 0>(S, P, tile, l0, l1, reference, ACCUM, sm,
-                                                   SplitStack{s_stack + threadIdx.x, stk}, t, r, s, ls, nn, nt);
-        else
-            stream_tile<COUNT, TWO, ACCUM ? 1 : 0>(S, P, tile, l0, l1, reference, ACCUM, sm, stk, t, r, s, ls, nn, nt);
+        auto walk = [&](auto stack) {
+            if constexpr (ONE)
+                stream_tile_one<COUNT, TWO, ACCUM ? 1 : 0>(S, P, tile, l0, l1, reference, ACCUM,
+                                                           sm.warp[threadIdx.x >> 5], stack, t, r, s, ls, nn, nt);
+            else
+                stream_tile<COUNT, TWO, ACCUM ? 1 : 0>(S, P, tile, l0, l1, reference, ACCUM, sm, stack, t, r, s, ls, nn, nt);
+        };
+        if constexpr (SHORT) walk(SplitStack{s_stack + threadIdx.x, stk});
+        else walk((uint2*)stk);
     }
     if (COUNT) { ls.nodes += nn; ls.tris += nt; }
     flush_stats(ls, P.stats);
 }
 
 // one-level kernels: the register cap as resident 128-thread blocks per SM
-// (5-8), or 8 with the first stack entries in shared memory; one ray per pixel and
-// light: 8 blocks, the stack in local memory
-template <bool ACCUM>
-static void* stream_kernel_flat(bool count, int minb, bool short_stack, bool one) {
-    if (one)
-        return count ? (void*)k_shadow_stream<true, ACCUM, 8, false, false, true>
-                     : (void*)k_shadow_stream<false, ACCUM, 8, false, false, true>;
+// (5-8), or 8 with the first stack entries in shared memory; the caller's choice, 8
+// without (one ray per light, 4K with 64 lights, shadow kernel at 5 / 6 / 7 / 8 / 8 with
+// shared entries: 98.3 / 90.3 / 88.1 / 89.7 / 90.2 ms; 1700x900 with 4: 1.13 / 1.06 /
+// 1.04 / 1.06 / 1.09 ms)
+template <bool ACCUM, bool ONE>
+static void* stream_kernel_flat(bool count, int minb, bool short_stack) {
     if (short_stack)
-        return count ? (void*)k_shadow_stream<true, ACCUM, 8, false, true>
-                     : (void*)k_shadow_stream<false, ACCUM, 8, false, true>;
-    if (minb >= 8) return count ? (void*)k_shadow_stream<true, ACCUM, 8> : (void*)k_shadow_stream<false, ACCUM, 8>;
-    if (minb == 7) return count ? (void*)k_shadow_stream<true, ACCUM, 7> : (void*)k_shadow_stream<false, ACCUM, 7>;
-    if (minb >= 6) return count ? (void*)k_shadow_stream<true, ACCUM, 6> : (void*)k_shadow_stream<false, ACCUM, 6>;
-    return count ? (void*)k_shadow_stream<true, ACCUM, 5> : (void*)k_shadow_stream<false, ACCUM, 5>;
+        return count ? (void*)k_shadow_stream<true, ACCUM, 8, false, true, ONE>
+                     : (void*)k_shadow_stream<false, ACCUM, 8, false, true, ONE>;
+    if (minb >= 8)
+        return count ? (void*)k_shadow_stream<true, ACCUM, 8, false, false, ONE>
+                     : (void*)k_shadow_stream<false, ACCUM, 8, false, false, ONE>;
+    if (minb == 7)
+        return count ? (void*)k_shadow_stream<true, ACCUM, 7, false, false, ONE>
+                     : (void*)k_shadow_stream<false, ACCUM, 7, false, false, ONE>;
+    if (minb >= 6)
+        return count ? (void*)k_shadow_stream<true, ACCUM, 6, false, false, ONE>
+                     : (void*)k_shadow_stream<false, ACCUM, 6, false, false, ONE>;
+    return count ? (void*)k_shadow_stream<true, ACCUM, 5, false, false, ONE>
+                 : (void*)k_shadow_stream<false, ACCUM, 5, false, false, ONE>;
 }
 
 }  // namespace hy

@@ -3,6 +3,7 @@
 
 namespace hy {
 void* stream_kernel_raw(bool count, int minb, bool short_stack, bool one) {
-    return stream_kernel_flat<false>(count, minb, short_stack, one);
+    return one ? stream_kernel_flat<false, true>(count, minb, short_stack)
+               : stream_kernel_flat<false, false>(count, minb, short_stack);
 }
 }  // namespace hy
