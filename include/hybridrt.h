@@ -197,12 +197,15 @@ typedef struct HyPassConfig {
                                2..32, each lane traces spp / group_lanes samples in turn);
                                0 = the next power of two >= spp */
     uint32_t min_blocks;    /* shadow-kernel variant: compiled for 5 (96 registers) or 8 (64 registers)
-                               resident 128-thread blocks per SM, the lane-group kernel also for 6
-                               and 7, a batch's tile-stream kernel for 6 (80) and 8 (64);
-                               0 = 6 for the lane-group kernel, 8 otherwise */
+                               resident 128-thread blocks per SM, the lane-group kernel and the
+                               one-level single-view tile streams also for 6 (80) and 7 (72), a
+                               batch's tile-stream kernel for 6 and 8; two-level tile streams: 8
+                               whatever is set.  The path trace: 3, 4, 5, 6 or 8 (below 3: uncapped).
+                               0 = 6 for the lane groups and the path trace, 8 otherwise */
     uint32_t visits_per_round; /* BVH node visits a shadow lane makes between two scheduling rounds
-                                  of the persistent shadow kernels (1..16; a lane whose ray ends
-                                  early waits for the round); 0 = 4, 32 in counting launches */
+                                  of the persistent shadow kernels (a lane whose ray ends early waits
+                                  for the round): 1..16, larger values taken as 16; 0 = 4, and 32 for
+                                  the tile streams of a counting launch, which test triangles at once */
 } HyPassConfig;
 
 typedef struct HyStats {
