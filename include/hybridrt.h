@@ -212,8 +212,11 @@ typedef struct HyStats {
     uint64_t shadow_rays;       /* rays traced by the shadow pass */
     uint64_t reflection_rays;   /* closest-hit bounce rays of mirror/glass pixels */
     uint64_t hit_shadow_rays;   /* shadow rays cast from bounce hit points */
-    uint64_t nodes_visited;     /* with HY_FLAG_COUNT_TRAVERSAL */
-    uint64_t tris_tested;       /* with HY_FLAG_COUNT_TRAVERSAL */
+    /* with HY_FLAG_COUNT_TRAVERSAL: the counts of each ray's own walk, shadow rays in the order
+     * that hy_scene_anyhit_order reports, which HY_ANYHIT_AUTO makes another one than the
+     * uncounted shadow pass's for a one-level structure beyond L2 (see below) */
+    uint64_t nodes_visited;
+    uint64_t tris_tested;
     uint32_t error_flags;       /* HY_STATUS_* */
     uint32_t _pad;
 } HyStats;
@@ -353,20 +356,23 @@ int hy_bvh_download_instances(HyCtx* ctx, float* records, float* boxes);
  *                        starts on a surface and meets its occluders away
  *                        from it, so fewer node visits;
  *   HY_ANYHIT_NEAR_FIRST front to back: a tile's rays to successive lights
- *                        start at the same nodes, the better order when the
- *                        structure does not fit in L2 and node fetches go to
- *                        DRAM;
+ *                        start at the same nodes, the better order for the
+ *                        shade and path-trace kernels when the structure does
+ *                        not fit in L2 and node fetches go to DRAM;
  *   HY_ANYHIT_AUTO       (default) far first for a one-level structure whose
  *                        nodes and leaf records fit in the device's L2, near
- *                        first otherwise (two-level structures included); the
- *                        default shadow schedule of an uncounted, unbatched
- *                        pass takes far first for every one-level structure.
- * The order is a property of the scene: it applies to every pass on it,
- * batched views included.  hy_scene_anyhit_order reports the order a pass
- * uses now (HY_ERR_NOT_READY without a built structure; under AUTO the order
- * of ray queries and counted passes).  Which triangle an
- * any-hit query reports can differ between the orders; whether it hits
- * cannot. */
+ *                        first otherwise (two-level structures included), but
+ *                        the default shadow schedule of an uncounted,
+ *                        unbatched pass goes far first through every one-level
+ *                        structure.
+ * The setting is a property of the scene: FAR_FIRST and NEAR_FIRST apply to
+ * every pass on it, batched views included.  hy_scene_anyhit_order reports
+ * the set order, or the one that AUTO takes for ray queries, counted passes,
+ * batched views, shading and path tracing (HY_ERR_NOT_READY without a built
+ * structure).  Beyond L2 a counted shadow pass under AUTO therefore counts the
+ * near-first walk; set FAR_FIRST for the counts of the walk that an uncounted
+ * one makes.  Which triangle an any-hit query reports can differ between the
+ * orders; whether it hits cannot. */
 enum { HY_ANYHIT_AUTO = 0, HY_ANYHIT_FAR_FIRST = 1, HY_ANYHIT_NEAR_FIRST = 2 };
 int hy_scene_set_anyhit_order(HyCtx* ctx, uint32_t order);
 int hy_scene_anyhit_order(HyCtx* ctx, uint32_t* resolved);

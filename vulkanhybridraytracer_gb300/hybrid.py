@@ -157,7 +157,8 @@ class HybridContext:
         L.check(self.lib.hy_scene_set_anyhit_order(self.h, order), "set_anyhit_order")
 
     def anyhit_order(self) -> int:
-        """The order passes use now: HY_ANYHIT_FAR_FIRST or HY_ANYHIT_NEAR_FIRST."""
+        """The set order, or under HY_ANYHIT_AUTO that of ray queries, counted passes, batches, shading and path
+        tracing: HY_ANYHIT_FAR_FIRST or HY_ANYHIT_NEAR_FIRST (hybridrt.h has the shadow schedule's rule)."""
         v = C.c_uint32()
         L.check(self.lib.hy_scene_anyhit_order(self.h, C.byref(v)), "anyhit_order")
         return int(v.value)
