@@ -735,8 +735,9 @@ __global__ void __launch_bounds__(32 * kSmallWarps) k_sah_small(const SahRange* 
 }
 
 // ---- one thread per range of 2 .. kTiny triangles ------------------------------
-// Nine of ten internal nodes lie in such subtrees, and a warp with bins per range
-// spent about 2,000 instructions on each.  Here the triangles sit in the thread's
+// Five of six internal nodes lie in such subtrees (83 % in the 1.5M-triangle scene, 82 in
+// one of 5k; at most 7 of 8 can), and a warp with bins per range spent about 2,000
+// instructions on each.  Here the triangles sit in the thread's
 // local array, their order in the nibbles of one word, and only the splits after an
 // occupied bin are tried: any other split parts the range like the one after the
 // last occupied bin before it, which comes first and so wins.  The same cost
