@@ -355,7 +355,9 @@ struct ProfScope {
 // structure far first here, also one beyond L2: the kernel keeps enough walks in
 // flight per SM for the fewer visits to pay although their fetches go to DRAM
 // (far / near, 7.3M triangles in 440 MB: 4K with 64 lights, one ray each, 105.2 /
-// 123.9 ms; 1080p with 16 lights 6.85 / 7.47, with 4 samples 18.5 / 20.8).  The shade
+// 123.9 ms; 1080p with 16 lights 6.85 / 7.47, with 4 samples 18.5 / 20.8; 1080p, 4 lights x
+// 16 samples over 3.9M / 5.9M / 6.6M / 9.0M triangles 18.4 / 19.7, 16.7 / 18.5, 10.9 /
+// 11.0, 15.4 / 16.9, with one ray per light 2.00 / 2.16, 1.78 / 1.97, 1.10 / 1.13, 1.71 / 1.82).  The shade
 // (3.70 / 3.51) and path-trace (7.55 / 7.39) kernels there and two-level structures
 // (10 MB of instance records and 1,025 instances 12.8 / 10.9) keep their order.  Counted
 // passes walk in the order that hy_scene_anyhit_order reports.
