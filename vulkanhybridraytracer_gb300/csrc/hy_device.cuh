@@ -606,7 +606,10 @@ __device__ __forceinline__ bool two_level_settle(const SceneDev& S, const RW& rw
 // the same node visits and triangle tests, in the same order, as a walk that
 // tests each node's triangles at once.
 // TWO: the two-level structure (r is the world ray; t.cur the current one).
-template <bool ANY, bool COUNT, bool TWO = false, class Stack = uint2*, class RW = RayPre, class Status = uint32_t*>
+// CMP: boxes accepted by comparisons, for the intervals that the signs of differences do
+// not hold for (signs_hold).
+template <bool ANY, bool COUNT, bool TWO = false, bool CMP = false, class Stack = uint2*, class RW = RayPre,
+          class Status = uint32_t*>
 __device__ __forceinline__ bool trav_node(const SceneDev& S, const RW& rw, float tmin, Trav& t, Stack stk,
                                           uint32_t& nodes_ctr, Status status) {
     if (++t.iters > S.max_iters) { raise_status(status, HY_STATUS_TIMEOUT); return true; }
@@ -661,9 +664,9 @@ __device__ __forceinline__ bool trav_node(const SceneDev& S, const RW& rw, float
     }
     const uint32_t q[3][4] = {{q2.x, q2.y, q2.z, q2.w}, {q3.x, q3.y, q3.z, q3.w}, {q4.x, q4.y, q4.z, q4.w}};
     // A box is hit when max(tn, tmin) <= rn(min(tf, tmax) * c).  rn(. * c) is
-    // monotone, so that is tn <= rn(tf c), tn <= rn(tmax c), tmin <= rn(tf c) (a
-    // ray has tmin <= tmax): three differences, product minus left-hand side, whose
-    // sign bits are gathered by one three-input OR and one funnel shift per slot.
+    // monotone, so that is tn <= rn(tf c), tn <= rn(tmax c), tmin <= rn(tf c), and tmin <=
+    // rn(tmax c), which signs_hold took care of: three differences, product minus
+    // left-hand side, whose sign bits are gathered by one three-input OR and one funnel shift per slot.
     // The differences run on the FMA pipe; min / max / compare would run on the ALU
     // pipe, which limits the walk.  Terms that differ give a difference of the right
     // sign, equal ones +0, except (-0) - (+0) = -0: the products are fmas with +0, which
@@ -685,6 +688,15 @@ __device__ __forceinline__ bool trav_node(const SceneDev& S, const RW& rw, float
             h2_to_f2(__byte_perm(q[a][j], 0u, sel[a] + 0x0202u), n1, f1);
             f2_unpack(f2_fma(f2_pack(n0, f0), adj2[a], org2[a]), tn[0][a], tf[0][a]);
             f2_unpack(f2_fma(f2_pack(n1, f1), adj2[a], org2[a]), tn[1][a], tf[1][a]);
+        }
+        if constexpr (CMP) {
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const float tnear = fmaxf(fmax3(tn[h][0], tn[h][1], tn[h][2]), tmin);
+                const float tfar = fminf(fmin3(tf[h][0], tf[h][1], tf[h][2]), t.tmax);
+                miss |= (tnear <= __fmul_rn(tfar, kBoxSlack) ? 0u : 1u) << (2 * j + h);
+            }
+            continue;
         }
         // both slots' products and differences as f32x2 (tnear * -1 + m is m - tnear)
         const unsigned long long near2 = f2_pack(fmax3(tn[0][0], tn[0][1], tn[0][2]), fmax3(tn[1][0], tn[1][1], tn[1][2]));
@@ -746,23 +758,32 @@ __device__ __forceinline__ bool trav_tri(const SceneDev& S, const RW& rw, float 
 
 // One node visit and then its triangles (the walk of a single ray).
 // Returns true when the ray is finished: t.h holds the hit, or id HY_NO_HIT.
-template <bool ANY, bool COUNT, bool TWO = false, class Stack = uint2*, class RW = RayPre>
+template <bool ANY, bool COUNT, bool TWO = false, bool CMP = false, class Stack = uint2*, class RW = RayPre>
 __device__ __forceinline__ bool trav_step(const SceneDev& S, const RW& rw, float tmin, Trav& t, Stack stk,
                                           uint32_t& nodes_ctr, uint32_t& tris_ctr, uint32_t* status) {
-    if (trav_node<ANY, COUNT, TWO>(S, rw, tmin, t, stk, nodes_ctr, status)) return true;
+    if (trav_node<ANY, COUNT, TWO, CMP>(S, rw, tmin, t, stk, nodes_ctr, status)) return true;
     while (t.pend_bits)
         if (trav_tri<ANY, COUNT, TWO>(S, rw, tmin, t, tris_ctr, status)) return true;
     return false;
 }
 
-template <bool ANY, bool COUNT, bool TWO = false>
+// Whether the signs of trav_node's differences accept the boxes that comparisons do for a
+// ray of this interval: it is not empty (up to the slack), has no NaN end, and, for a
+// closest hit, cannot become empty as tmax shrinks to a negative distance.  The rays
+// that the passes trace themselves have tmin = 0.001 and tmax >= 1.
+template <bool ANY>
+__device__ __forceinline__ bool signs_hold(float tmin, float tmax) {
+    return tmin <= __fmul_rn(tmax, kBoxSlack) && (ANY || tmin >= 0.f);
+}
+
+template <bool ANY, bool COUNT, bool TWO = false, bool CMP = false>
 __device__ __forceinline__ Hit traverse(const SceneDev& S, const RayPre& r, float tmin, float tmax,
                                         uint32_t* nodes_ctr, uint32_t* tris_ctr, uint32_t* status) {
     uint2 stk[kStackMax];
     Trav t;
     trav_init(t, r, tmax);
     uint32_t nn = 0, nt = 0;
-    while (!trav_step<ANY, COUNT, TWO>(S, r, tmin, t, stk, nn, nt, status)) {
+    while (!trav_step<ANY, COUNT, TWO, CMP>(S, r, tmin, t, stk, nn, nt, status)) {
     }
     if (COUNT) { *nodes_ctr += nn; *tris_ctr += nt; }
     return t.h;

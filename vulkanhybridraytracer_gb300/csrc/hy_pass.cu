@@ -549,10 +549,19 @@ __global__ void __launch_bounds__(128, 8) k_trace(const SceneDev S, const HyRay*
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i - threadIdx.x < n; i += gridDim.x * blockDim.x) {
         if (i < n) {
             HyRay r = rays[i];
-            // an empty interval enters no box (the walk's box test takes tmin <= tmax for granted)
-            const float tmax = r.tmin > __fmul_rn(r.tmax, kBoxSlack) ? -INFINITY : r.tmax;
-            Hit h = trace<ANY, COUNT>(S, mk(r.org[0], r.org[1], r.org[2]), mk(r.dir[0], r.dir[1], r.dir[2]), r.tmin,
-                                      tmax, ls, status);
+            Hit h;
+            if (signs_hold<ANY>(r.tmin, r.tmax)) {
+                h = trace<ANY, COUNT>(S, mk(r.org[0], r.org[1], r.org[2]), mk(r.dir[0], r.dir[1], r.dir[2]), r.tmin,
+                                      r.tmax, ls, status);
+            } else {
+                const CountedHit c =
+                    S.two_level ? traverse_compared<ANY, COUNT, true>(S, mk(r.org[0], r.org[1], r.org[2]),
+                                                                      mk(r.dir[0], r.dir[1], r.dir[2]), r.tmin, r.tmax, status)
+                                : traverse_compared<ANY, COUNT, false>(S, mk(r.org[0], r.org[1], r.org[2]),
+                                                                       mk(r.dir[0], r.dir[1], r.dir[2]), r.tmin, r.tmax, status);
+                h = c.h;
+                if (COUNT) { ls.nodes += c.nodes; ls.tris += c.tris; }
+            }
             ls.shadow++;
             HyHit o;
             o.t = h.id == HY_NO_HIT ? 0.f : h.t;
@@ -603,9 +612,12 @@ __global__ void __launch_bounds__(128, 8) k_trace_closest(const SceneDev S, cons
                 i = mine;
                 const float4 a = __ldg((const float4*)(rays + i)), b = __ldg((const float4*)(rays + i) + 1);
                 tmin = a.w;
-                // an empty interval enters no box (the walk's box test takes tmin <= tmax for granted)
-                const float tmax = tmin > __fmul_rn(b.w, kBoxSlack) ? -INFINITY : b.w;
-                closest_start<TWO>(w, t, r, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), tmin, tmax);
+                // as for any hit: an interval that becomes empty behind the origin costs this
+                // walk node visits, which it does not report, and changes no hit
+                if (signs_hold<true>(tmin, b.w))
+                    closest_start<TWO>(w, t, r, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), tmin, b.w);
+                else
+                    t.tmax = NAN;  // not a ray for this walk (one of its rays never has a NaN end)
                 live = true;
             }
         }
@@ -614,13 +626,13 @@ __global__ void __launch_bounds__(128, 8) k_trace_closest(const SceneDev S, cons
             continue;
         }
         uint32_t limits = 0;
-        const bool over = closest_round<TWO>(S, w, live, tmin, (uint2*)stk, t, r, limits, status);
-        if (live && over) {
-            if (limits) {  // a limit ran out: the plain walk decides
-                const float4 d = w.ray[lane];
+        const bool alone = live && t.tmax != t.tmax;
+        const bool over = closest_round<TWO>(S, w, live && !alone, tmin, (uint2*)stk, t, r, limits, status);
+        if (alone || (live && over)) {
+            if (alone || limits) {  // or a limit ran out: the plain walk decides
                 const HyRay& q = rays[i];
-                const float tmax = q.tmin > __fmul_rn(q.tmax, kBoxSlack) ? -INFINITY : q.tmax;
-                t.h = traverse_again<TWO>(S, mk(q.org[0], q.org[1], q.org[2]), mk(d.x, d.y, d.z), q.tmin, tmax, status);
+                t.h = traverse_compared<false, false, TWO>(S, mk(q.org[0], q.org[1], q.org[2]),
+                                                           mk(q.dir[0], q.dir[1], q.dir[2]), q.tmin, q.tmax, status).h;
             }
             const bool hit = t.h.id != HY_NO_HIT;
             reinterpret_cast<float4*>(hits)[i] = make_float4(hit ? t.h.t : 0.f, __uint_as_float(t.h.id),

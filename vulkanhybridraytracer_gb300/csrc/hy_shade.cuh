@@ -42,11 +42,20 @@ __device__ __forceinline__ Hit trace(const SceneDev& S, f3 o, f3 d, float tmin, 
     return h;
 }
 
-// a ray by itself, out of line: for the rays whose walk ran into a limit
-template <bool TWO>
-__device__ __noinline__ Hit traverse_again(const SceneDev& S, f3 o, f3 d, float tmin, float tmax, uint32_t* status) {
-    uint32_t nn = 0, nt = 0;
-    return traverse<false, false, TWO>(S, ray_pre(o, d), tmin, tmax, &nn, &nt, status);
+// a ray by itself, out of line, its boxes accepted by comparisons: for the intervals that
+// signs do not hold for, and for rays whose walk among others ran into a limit.  Counted
+// closest-hit queries with tmin < 0 are slower for it (2M over 1.5M triangles 932 -> 982 us,
+// two levels 1283 -> 1360); everything else measured as without it.
+struct CountedHit {
+    Hit h;
+    uint32_t nodes, tris;
+};
+template <bool ANY, bool COUNT, bool TWO>
+__device__ __noinline__ CountedHit traverse_compared(const SceneDev& S, f3 o, f3 d, float tmin, float tmax,
+                                                     uint32_t* status) {
+    CountedHit c{};
+    c.h = traverse<ANY, COUNT, TWO, true>(S, ray_pre(o, d), tmin, tmax, &c.nodes, &c.tris, status);
+    return c;
 }
 
 // equirect NEAREST / REPEAT lookup of an RGBA8 map.  One copy for all callers (the
