@@ -21,6 +21,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "hy_device.cuh"
@@ -664,7 +665,8 @@ __global__ void __launch_bounds__(kClimb) k_climb(const uint32_t* __restrict__ o
 // plan: 8 BVH2 refs per node in slot order (0xffffffff = empty).  Eight lanes per
 // node: the first spreads the node's 8 slots over its subtree by the slot budgets,
 // then lane i holds child i and its cost in each slot, and each of the assignment's
-// steps takes the best (cost, then lowest child, then lowest slot) over the lanes.
+// steps takes the best (cost, then lowest child, then lowest slot) over the lanes, the
+// choice of a search through children and slots in order that a greater cost renews.
 // counts[k]: (child nodes << 32) | leaf triangles.  (A thread per node with its 8 x 8
 // costs in local memory: 651 us for the 171k nodes of 1.5M triangles.)
 __global__ void __launch_bounds__(128) k_collapse_plan(const uint32_t* __restrict__ lvl, uint32_t m,
@@ -728,29 +730,47 @@ __global__ void __launch_bounds__(128) k_collapse_plan(const uint32_t* __restric
     uint32_t taken = 0;  // slots
     int slot = -1;       // this lane's
     const int steps = __reduce_max_sync(0xffffffffu, nc);
-    for (int it = 0; it < steps; it++) {
-        // this child's best free slot, first of equals
-        int bs = -1;
-        float bc = 0.f;
-        if (has && slot < 0) {
+    // NANS: a NaN cost (centroids beyond float) is never greater, so it is a step's choice only
+    // where it comes first of all
+    auto assign = [&](auto nans) {
+        constexpr bool NANS = decltype(nans)::value;
+        for (int it = 0; it < steps; it++) {
+            // this child's best free slot, first of equals
+            const bool open = has && slot < 0;
+            const int first = __ffs(~taken) - 1;
+            bool nan_first = false;
+            int bs = -1;
+            float bc = 0.f;
+            if (open) {
 #pragma unroll
-            for (int sl = 0; sl < 8; sl++)
-                if (!((taken >> sl) & 1u) && (bs < 0 || cost[sl] > bc)) { bs = sl; bc = cost[sl]; }
-        }
-        // the group's best child, in order: only a strictly greater cost wins
-        int who = -1, ws = -1;
-        float wc = 0.f;
+                for (int sl = 0; sl < 8; sl++) {
+                    if ((taken >> sl) & 1u) continue;
+                    if (NANS && sl == first) nan_first = cost[sl] != cost[sl];
+                    if (bs < 0 ? !NANS || cost[sl] >= -INFINITY : cost[sl] > bc) { bs = sl; bc = cost[sl]; }
+                }
+            }
+            // the group's best child, in order: only a strictly greater cost wins
+            int who = -1, ws = -1;
+            float wc = 0.f;
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const int os = __shfl_sync(0xffffffffu, bs, g0 + i);
-            const float oc = __shfl_sync(0xffffffffu, bc, g0 + i);
-            if (os >= 0 && (who < 0 || oc > wc)) { who = i; ws = os; wc = oc; }
+            for (int i = 0; i < 8; i++) {
+                const int os = __shfl_sync(0xffffffffu, bs, g0 + i);
+                const float oc = __shfl_sync(0xffffffffu, bc, g0 + i);
+                if (os >= 0 && (who < 0 || oc > wc)) { who = i; ws = os; wc = oc; }
+            }
+            if (NANS) {
+                const uint32_t opens = (__ballot_sync(0xffffffffu, open) >> g0) & 0xffu;
+                const uint32_t firsts = (__ballot_sync(0xffffffffu, nan_first) >> g0) & 0xffu;
+                if (firsts & opens & (0u - opens)) { who = __ffs(opens) - 1; ws = first; }
+            }
+            if (who >= 0) {
+                taken |= 1u << ws;
+                if (who == (int)li) slot = ws;
+            }
         }
-        if (who >= 0) {
-            taken |= 1u << ws;
-            if (who == (int)li) slot = ws;
-        }
-    }
+    };
+    if (__any_sync(0xffffffffu, !(fabsf(dd[0]) + fabsf(dd[1]) + fabsf(dd[2]) < INFINITY))) assign(std::true_type{});
+    else assign(std::false_type{});
     uint32_t at = 0xffffffffu;  // the child in slot li
 #pragma unroll
     for (int i = 0; i < 8; i++) {
