@@ -112,3 +112,30 @@ def test_hits_at_a_negative_start(gpu_lib, oracle_lib):
         assert np.array_equal(ctx.trace(dev, False)[0].cpu().numpy().view(np.uint32), want.view(np.uint32))
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("length", [3e38, 1e30, 2.0 ** 41, 2.0 ** 39, 2.0 ** -39, 2.0 ** -41, 1e-21, 1e-38])
+@pytest.mark.parametrize("instanced", [False, True])
+def test_direction_lengths(gpu_lib, oracle_lib, instanced, length):
+    """Closest hits along directions so long or short that distances underflow or box and
+    triangle distances part: the queries without counters give the plain walk's hits."""
+    import torch
+    from vulkanhybridraytracer_gb300 import scenes
+    from vulkanhybridraytracer_gb300.hybrid import HybridContext
+    n, rng = 200_000, np.random.default_rng(2)
+    rays = np.zeros((n, 8), np.float32)
+    rays[:, 0:3] = rng.uniform([-10, -1, -10], [10, 5, 10], (n, 3))
+    d = rng.uniform(-1, 1, (n, 3))
+    rays[:, 4:7] = d / np.abs(d).max(axis=1, keepdims=True) * length
+    rays[::2, 4] = rng.uniform(-0.5, 0.5, len(rays[::2]))
+    rays[:, 3], rays[:, 7] = rng.choice([0.0, -3e38, -np.inf], n), np.inf if length < 1e-35 else 1000.0 * max(1.0, 1.0 / length)
+    ctx = HybridContext(0)
+    try:
+        ctx.set_scene(scenes.diff(3, 64, 64).scene)
+        ctx.build_bvh(instanced=instanced)
+        dev = torch.from_numpy(rays).cuda()
+        plain, _ = ctx.trace(dev, False, count=True)
+        queued, _ = ctx.trace(dev, False)
+        assert torch.equal(plain.view(torch.int32), queued.view(torch.int32))
+    finally:
+        ctx.close()

@@ -613,8 +613,12 @@ __global__ void __launch_bounds__(128, 8) k_trace_closest(const SceneDev S, cons
                 const float4 a = __ldg((const float4*)(rays + i)), b = __ldg((const float4*)(rays + i) + 1);
                 tmin = a.w;
                 // as for any hit: an interval that becomes empty behind the origin costs this
-                // walk node visits, which it does not report, and changes no hit
-                if (signs_hold<true>(tmin, b.w))
+                // walk node visits, which it does not report, and changes no hit.  The box
+                // test's slack is relative: where distances are subnormal or the reciprocal of a
+                // vanishing direction is cut off, boxes are lost by how far the interval has
+                // shrunk, and the plain walk's order decides.
+                const float d = fmax3(fabsf(b.x), fabsf(b.y), fabsf(b.z));
+                if (signs_hold<true>(tmin, b.w) && d >= 0x1p-40f && d <= 0x1p40f)
                     closest_start<TWO>(w, t, r, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), tmin, b.w);
                 else
                     t.tmax = NAN;  // not a ray for this walk (one of its rays never has a NaN end)

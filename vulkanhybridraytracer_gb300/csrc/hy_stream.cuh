@@ -219,7 +219,8 @@ __device__ __forceinline__ RoundResult stream_round(const SceneDev& S, const Pas
 // hits meet in the owner's 64-bit key (distance, id; the lower id on equal
 // distances), and the pair whose key is left hands its distance and barycentrics
 // over.  The closest hit does not depend on the order of visits or on how early the
-// interval shrinks, so it is the plain walk's, bit for bit; a ray may make a few more
+// interval shrinks, so it is the plain walk's, bit for bit (rays for which the box test's
+// slack does not hold are not walked here: k_trace_closest); a ray may make a few more
 // node visits.  A ray that runs into a limit is walked anew by itself (plain), so
 // that the limit holds for the plain walk's visits.
 template <bool TWO>
