@@ -286,14 +286,13 @@ __global__ void k_scan64_apply(const unsigned long long* __restrict__ in, uint32
     if (!sums && threadIdx.x == 0) *total = tot;
 }
 
+// sums: room for one value per SCAN_TILE inputs
 static int scan_exclusive64(HyCtx* c, const unsigned long long* in, unsigned long long* out, uint32_t n,
-                            unsigned long long* d_total) {
+                            unsigned long long* sums, unsigned long long* d_total) {
     const uint32_t nb = std::max<uint32_t>((n + SCAN_TILE - 1) / SCAN_TILE, 1);
-    unsigned long long* sums = nullptr;
-    if (nb > 1) {
-        int rc = ctx_alloc(c, c->scan_tmp, (size_t)nb * 8);
-        if (rc) return rc;
-        sums = c->scan_tmp.as<unsigned long long>();
+    if (nb == 1) {
+        sums = nullptr;
+    } else {
         k_scan64_sums<<<nb, SCAN_T, 0, c->stream>>>(in, n, sums);
         k_scan64_top<<<1, SCAN_T, 0, c->stream>>>(sums, nb, d_total);
     }
@@ -1005,11 +1004,14 @@ static int build_core(HyCtx* c, uint32_t n, uint32_t node_off, uint32_t rec_off,
     unsigned long long* tot = c->total.as<unsigned long long>();
     unsigned long long* counts = c->ni.as<unsigned long long>();
     unsigned long long* scan = c->ni_scan.as<unsigned long long>();
+    // the sort's other key buffer, free by now: scan_tmp at 8 B a value would not fit budgets
+    // that it fits at 4
+    unsigned long long* sums = c->keys[cur ^ 1].as<unsigned long long>();
     while (m > 0) {
         const uint32_t* lvl = c->lvl_ref[lv].as<uint32_t>();
         k_collapse_plan<<<cdiv(m, 16), 128, 0, s>>>(lvl, m, bvh2, ord, c->tribox.as<float>(), c->dp_k.as<uint8_t>(),
                                                     c->plan.as<uint32_t>(), counts);
-        if ((rc = scan_exclusive64(c, counts, scan, m, tot))) return rc;
+        if ((rc = scan_exclusive64(c, counts, scan, m, sums, tot))) return rc;
         k_collapse_emit<<<cdiv(m, 128), 128, 0, s>>>(m, level_start, tri_start, node_off, rec_off, lvl,
                                                      c->plan.as<uint32_t>(), scan, bvh2, ord,
                                                      c->tribox.as<float>(), c->world.as<float4>(),
