@@ -784,12 +784,21 @@ int hy_trace_rays(HyCtx* c, const HyRay* rays, uint32_t n, int any_hit, HyHit* h
     int rc = reset_counters(c);
     if (rc) return rc;
     bool count = st != nullptr;
-    // queries that report no counts: 8 resident blocks per SM on the closest-hit queue
-    // (which loads and stores 16 bytes at a time)
-    const bool queued = !count && any_hit == 0 && n <= 0xfff00000u && ((uintptr_t)rays | (uintptr_t)hits) % 16 == 0;
+    // Closest-hit queries that report no counts: 8 resident blocks per SM on the queue (which
+    // loads and stores 16 bytes at a time), unless every ray has a lane of its own and walks
+    // end soon: then a round's bookkeeping is not paid back.  Kernel, plain / queue: 65,536
+    // rays over 5k triangles 18.7 / 22.7 us, two levels 26 / 38, over 82k 33.1 / 35.6 and 46 /
+    // 57, over 1.5M 67.8 / 69.1, over 1,025 instances of 148k records 274 / 304 (1,000 rays: 232 /
+    // 209), over 2.2M 143 / 122; 300,000 rays 38 / 36, 49 / 45, 68 / 55, 84 / 81, 165 / 112, 858 / 558, 451 / 255.
+    const uint64_t wave = 128ull * (uint32_t)c->num_sms;
+    const bool short_walks = c->n_records < 100000u && n <= 8 * wave;
+    const bool queued = !count && any_hit == 0 && !short_walks && n <= 0xfff00000u &&
+                        ((uintptr_t)rays | (uintptr_t)hits) % 16 == 0;
+    // two levels: the plain kernel at 5 resident blocks
+    const bool wide = short_walks || n <= 5 * wave;
     int grid = std::max(1, std::min<int>(c->num_sms * (queued ? 8 : 16), (int)((n + 127) / 128)));
     HY_CUDA_TRY(launch_trace(scene_dev(c), rays, n, any_hit != 0, count, hits, dev_stats(c), dev_status(c),
-                             queued ? dev_queue(c, WQ_MISC) : nullptr, grid, c->stream));
+                             queued ? dev_queue(c, WQ_MISC) : nullptr, wide, grid, c->stream));
     return finish_call(c, st, true);
 }
 

@@ -539,23 +539,27 @@ __global__ void __launch_bounds__(kBlurW * kBlurH) k_accumulate(const AccumParam
     }
 }
 
-// generic ray queries (32 B ray in, 16 B hit out), a thread per ray: any-hit ones (8
-// resident blocks: 2M incoherent rays 592 -> 461 us, the call), counting ones, and
-// buffers that are not 16-byte aligned
-template <bool ANY, bool COUNT>
-__global__ void __launch_bounds__(128, 8) k_trace(const SceneDev S, const HyRay* __restrict__ rays, uint32_t n,
-                                               HyHit* __restrict__ hits, unsigned long long* stats, uint32_t* status) {
+// generic ray queries (32 B ray in, 16 B hit out), a thread per ray: any-hit ones,
+// counting ones, buffers that are not 16-byte aligned, and closest hits of a launch too
+// small for the queue (hy_trace_rays).  LV 0: either level, 8 resident blocks (2M incoherent
+// any-hit rays 592 -> 461 us, the call).  LV 2: two levels at 5 blocks (96 registers), for
+// launches that are resident at once so: the spills at 8 cost such a launch 5 to 10 % (any-hit
+// rays over 1,025 instances, kernel at 5 / 8 blocks: 32,000 rays 97 / 106 us, 131,072 165 / 142).
+template <bool ANY, bool COUNT, int LV>
+__global__ void __launch_bounds__(128, LV == 2 ? 5 : 8) k_trace(const SceneDev S, const HyRay* __restrict__ rays,
+                                                                uint32_t n, HyHit* __restrict__ hits,
+                                                                unsigned long long* stats, uint32_t* status) {
     LaneStats ls;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i - threadIdx.x < n; i += gridDim.x * blockDim.x) {
         if (i < n) {
             HyRay r = rays[i];
             Hit h;
             if (signs_hold<ANY>(r.tmin, r.tmax)) {
-                h = trace<ANY, COUNT>(S, mk(r.org[0], r.org[1], r.org[2]), mk(r.dir[0], r.dir[1], r.dir[2]), r.tmin,
-                                      r.tmax, ls, status);
+                h = trace<ANY, COUNT, LV>(S, mk(r.org[0], r.org[1], r.org[2]), mk(r.dir[0], r.dir[1], r.dir[2]), r.tmin,
+                                          r.tmax, ls, status);
             } else {
                 const CountedHit c =
-                    S.two_level ? traverse_compared<ANY, COUNT, true>(S, mk(r.org[0], r.org[1], r.org[2]),
+                    LV == 2 || S.two_level ? traverse_compared<ANY, COUNT, true>(S, mk(r.org[0], r.org[1], r.org[2]),
                                                                       mk(r.dir[0], r.dir[1], r.dir[2]), r.tmin, r.tmax, status)
                                 : traverse_compared<ANY, COUNT, false>(S, mk(r.org[0], r.org[1], r.org[2]),
                                                                        mk(r.dir[0], r.dir[1], r.dir[2]), r.tmin, r.tmax, status);
@@ -1190,15 +1194,23 @@ cudaError_t launch_accumulate(const AccumParams& A, cudaStream_t s) {
     return cudaGetLastError();
 }
 
+template <bool ANY, bool COUNT>
+static void plain_queries(const SceneDev& S, const HyRay* rays, uint32_t n, HyHit* hits, unsigned long long* stats,
+                          uint32_t* status, bool wide, int grid, cudaStream_t s) {
+    if (wide && S.two_level) k_trace<ANY, COUNT, 2><<<grid, 128, 0, s>>>(S, rays, n, hits, stats, status);
+    else k_trace<ANY, COUNT, 0><<<grid, 128, 0, s>>>(S, rays, n, hits, stats, status);
+}
+
 cudaError_t launch_trace(const SceneDev& S, const HyRay* rays, uint32_t n, bool any, bool count, HyHit* hits,
-                         unsigned long long* stats, uint32_t* status, uint32_t* queue, int grid, cudaStream_t s) {
+                         unsigned long long* stats, uint32_t* status, uint32_t* queue, bool wide, int grid,
+                         cudaStream_t s) {
     if (n == 0) return cudaSuccess;
     if (any) {
-        if (count) k_trace<true, true><<<grid, 128, 0, s>>>(S, rays, n, hits, stats, status);
-        else k_trace<true, false><<<grid, 128, 0, s>>>(S, rays, n, hits, stats, status);
+        if (count) plain_queries<true, true>(S, rays, n, hits, stats, status, wide, grid, s);
+        else plain_queries<true, false>(S, rays, n, hits, stats, status, wide, grid, s);
     } else {
-        if (count) k_trace<false, true><<<grid, 128, 0, s>>>(S, rays, n, hits, stats, status);
-        else if (!queue) k_trace<false, false><<<grid, 128, 0, s>>>(S, rays, n, hits, stats, status);
+        if (count) plain_queries<false, true>(S, rays, n, hits, stats, status, wide, grid, s);
+        else if (!queue) plain_queries<false, false>(S, rays, n, hits, stats, status, wide, grid, s);
         else if (S.two_level) k_trace_closest<true><<<grid, 128, 0, s>>>(S, rays, n, hits, queue, status);
         else k_trace_closest<false><<<grid, 128, 0, s>>>(S, rays, n, hits, queue, status);
     }

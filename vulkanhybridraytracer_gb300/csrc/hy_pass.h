@@ -112,7 +112,8 @@ cudaError_t launch_accumulate(const AccumParams& A, cudaStream_t s);
 cudaError_t launch_post(const uint8_t* in_bgra8, const float* in_rgba32f, uint32_t n, uint8_t* out_bgra8,
                         cudaStream_t s);
 cudaError_t launch_trace(const SceneDev& S, const HyRay* rays, uint32_t n, bool any, bool count, HyHit* hits,
-                         unsigned long long* stats, uint32_t* status, uint32_t* queue, int grid, cudaStream_t s);
+                         unsigned long long* stats, uint32_t* status, uint32_t* queue, bool wide, int grid,
+                         cudaStream_t s);
 cudaError_t launch_gbuffer(const SceneDev& S, const GbufParams& G, cudaStream_t s);
 // batches: block / shortd are the tile-stream kernel's threads per block and
 // shared stack entries (the shade and lane-group kernels: 128 / 0)
