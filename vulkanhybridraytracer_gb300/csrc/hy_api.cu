@@ -817,7 +817,7 @@ int hy_gbuffer_primary(HyCtx* c, const HyCamera* cam, uint32_t W, uint32_t H, fl
     std::memcpy(G.inv_proj, cam->inv_proj, 64);
     for (int i = 0; i < 6; i++) G.planes[i] = planes[i];
     G.status = dev_status(c);
-    HY_CUDA_TRY(launch_gbuffer(scene_dev(c), G, c->stream));
+    HY_CUDA_TRY(launch_gbuffer(scene_dev(c), G, c->num_sms, c->stream));
     return finish_call(c, nullptr, true);
 }
 

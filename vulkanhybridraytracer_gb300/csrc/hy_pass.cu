@@ -666,11 +666,15 @@ __device__ __forceinline__ f3 mat_vec3(const float* m, float x, float y, float z
 
 // A warp per 8x4 tile; compiled per structure level, each with one copy of the walk, for
 // 8 resident blocks (1080p, the call: 16x2 texels a warp, 94 registers 458 us; 8x4 tiles
-// at 1 / 6 / 8 / 10 / 12 blocks 434 / 409 / 385 / 394 / 409).
-template <bool TWO>
-__global__ void __launch_bounds__(128, 8) k_gbuffer(const SceneDev S, const GbufParams G) {
+// at 1 / 6 / 8 / 10 / 12 blocks 434 / 409 / 385 / 394 / 409).  SMALL: two-level frames of a few
+// resident launches, where the spills and the tiles' longer slowest walks cost more than
+// residency gives: 5 blocks (93 registers, no spills; uncapped it takes 102, 4 blocks),
+// 16x2 texels a warp.
+template <bool TWO, bool SMALL = false>
+__global__ void __launch_bounds__(128, SMALL ? 5 : 8) k_gbuffer(const SceneDev S, const GbufParams G) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t x = blockIdx.x * 16 + (warp & 1) * 8 + (lane & 7), y = blockIdx.y * 8 + (warp >> 1) * 4 + (lane >> 3);
+    const uint32_t x = blockIdx.x * 16 + (SMALL ? lane & 15 : (warp & 1) * 8 + (lane & 7));
+    const uint32_t y = blockIdx.y * 8 + (SMALL ? warp * 2 + (lane >> 4) : (warp >> 1) * 4 + (lane >> 3));
     if (x >= G.W || y >= G.H) return;
     size_t i = (size_t)y * G.W + x;
     float ux = __fdiv_rn(__fadd_rn((float)x, 0.5f), (float)G.W), uy = __fdiv_rn(__fadd_rn((float)y, 0.5f), (float)G.H);
@@ -1217,9 +1221,14 @@ cudaError_t launch_trace(const SceneDev& S, const HyRay* rays, uint32_t n, bool 
     return cudaGetLastError();
 }
 
-cudaError_t launch_gbuffer(const SceneDev& S, const GbufParams& G, cudaStream_t s) {
+// SMALL, in two levels: up to 6 launches of 5 resident blocks per SM.  Kernel, SMALL / 8 blocks on
+// tiles, 1,025 instances: 320x240 315 / 359 us, 640x360 335 / 408, 800x450 394 / 423, 960x540 503 /
+// 486, 1280x720 762 / 690; 1.5M triangles in 49 instances 120 / 128, 143 / 172, 147 / 158,
+// 175 / 190, 254 / 239.
+cudaError_t launch_gbuffer(const SceneDev& S, const GbufParams& G, int num_sms, cudaStream_t s) {
     dim3 g((G.W + 15) / 16, (G.H + 7) / 8);
-    if (S.two_level) k_gbuffer<true><<<g, 128, 0, s>>>(S, G);
+    if (S.two_level && (uint64_t)G.W * G.H <= 6ull * 5 * 128 * (uint32_t)num_sms) k_gbuffer<true, true><<<g, 128, 0, s>>>(S, G);
+    else if (S.two_level) k_gbuffer<true><<<g, 128, 0, s>>>(S, G);
     else k_gbuffer<false><<<g, 128, 0, s>>>(S, G);
     return cudaGetLastError();
 }
