@@ -1227,7 +1227,8 @@ cudaError_t launch_trace(const SceneDev& S, const HyRay* rays, uint32_t n, bool 
 // 175 / 190, 254 / 239.
 cudaError_t launch_gbuffer(const SceneDev& S, const GbufParams& G, int num_sms, cudaStream_t s) {
     dim3 g((G.W + 15) / 16, (G.H + 7) / 8);
-    if (S.two_level && (uint64_t)G.W * G.H <= 6ull * 5 * 128 * (uint32_t)num_sms) k_gbuffer<true, true><<<g, 128, 0, s>>>(S, G);
+    const uint64_t small = 6ull * 5 * 128 * (uint32_t)num_sms;
+    if (S.two_level && (uint64_t)G.W * G.H <= small) k_gbuffer<true, true><<<g, 128, 0, s>>>(S, G);
     else if (S.two_level) k_gbuffer<true><<<g, 128, 0, s>>>(S, G);
     else k_gbuffer<false><<<g, 128, 0, s>>>(S, G);
     return cudaGetLastError();
